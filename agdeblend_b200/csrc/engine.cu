@@ -170,7 +170,7 @@ int agd_gpu_problem_info(agd_gpu_problem const *pb, long int *info) {
   for (int c : e.win_class) n_fast += c >= 0 ? 1 : 0;
   const long nw = (long)e.plan.windows.size();
   info[8] = (nw > 0 && n_fast == nw) ? 1 : (n_fast > 0 ? 2 : 0);
-  info[9] = e.wav_fast ? 1 : 0;
+  info[9] = e.wav_fast && !e.wav_padded ? 1 : 0;
   info[10] = e.classes.empty() ? -1 : e.classes[0]->fwd_pick;
   info[11] = e.classes.empty() ? -1 : e.classes[0]->adj_pick;
   info[12] = e.classes.empty() ? 0 : (long)e.classes[0]->fwd_vars.size();

@@ -166,9 +166,10 @@ class Engine {
   bool multi = false;
   std::vector<R> steps;        // per problem
   DevArray<R> step_dev, pmax;  // per problem
-  // prime-factor wavelet kernel (wavelet_fast.cuh), used when every window's
-  // trace length factors into supported coprime prime powers
-  bool wav_fast = false;
+  // prime-factor wavelet kernel (wavelet_fast.cuh); wav_padded: some trace
+  // length does not factor into supported coprime prime powers and is
+  // zero-padded to one that does
+  bool wav_fast = false, wav_padded = false;
   DevArray<WaveletFastJob<R>> wavf_jobs;
   DevArray<unsigned short> pfa_map;  // per trace length: qmap [C], kpos [C]
   TimeLaunch wavf;
@@ -230,16 +231,22 @@ class Engine {
     smem_max = std::min({opt_in(axis_pass<R>, limit), opt_in(time_c2r_ola<R>, limit),
                          opt_in(time_r2c<R>, limit), opt_in(wavelet_apply<R>, limit),
                          opt_in(line_dft_fwd<R>, limit), opt_in(line_dft_adj<R>, limit)});
+    opt_in_wavelet<false>(limit);
+    opt_in_wavelet<true>(limit);
+  }
+
+  template <bool PAD>
+  void opt_in_wavelet(int limit) {
     if constexpr (sizeof(R) == sizeof(float))
-      smem_max = std::min({smem_max, opt_in(wavelet_fast<R, 2, 17>, limit),
-                           opt_in(wavelet_fast<R, 3, 17>, limit),
-                           opt_in(wavelet_fast<R, 4, 17>, limit),
-                           opt_in(wavelet_fast<R, 2, 32>, limit),
-                           opt_in(wavelet_fast<R, 3, 32>, limit)});
+      smem_max = std::min({smem_max, opt_in(wavelet_fast<R, 2, 17, PAD>, limit),
+                           opt_in(wavelet_fast<R, 3, 17, PAD>, limit),
+                           opt_in(wavelet_fast<R, 4, 17, PAD>, limit),
+                           opt_in(wavelet_fast<R, 2, 32, PAD>, limit),
+                           opt_in(wavelet_fast<R, 3, 32, PAD>, limit)});
     else
-      smem_max = std::min({smem_max, opt_in(wavelet_fast<R, 1, 17>, limit),
-                           opt_in(wavelet_fast<R, 2, 17>, limit),
-                           opt_in(wavelet_fast<R, 1, 32>, limit)});
+      smem_max = std::min({smem_max, opt_in(wavelet_fast<R, 1, 17, PAD>, limit),
+                           opt_in(wavelet_fast<R, 2, 17, PAD>, limit),
+                           opt_in(wavelet_fast<R, 1, 32, PAD>, limit)});
   }
 
   // twiddle tables of the register DFTs in constant memory of the current
@@ -279,13 +286,63 @@ class Engine {
         return false;
       sh.f[sh.nf++] = q;
     }
+    pfa_strides(sh);
+    return true;
+  }
+
+  static void pfa_strides(PfaShape &sh) {
     int g = 1;
     for (int i = sh.nf - 1; i >= 0; --i) {
       sh.g[i] = g;
       sh.inv_g[i] = 1.0f / (float)g;
-      sh.inv_lines[i] = (float)sh.f[i] / (float)N;
+      sh.inv_lines[i] = (float)sh.f[i] / (float)sh.N;
       g *= sh.f[i];
     }
+  }
+
+  // The transform length N >= 2 C - 1 for a zero-padded trace: the product
+  // of at most kPfaMaxFactors pairwise coprime prime powers up to 17 (whose
+  // register DFTs fit 64 registers) with the least arithmetic per transform.
+  // The operation counts are those of the register DFTs, plus kPass per
+  // point for the shared-memory round trip of a pass; a power of two costs
+  // the least per point, so lengths with a factor 16 win where one is near.
+  static bool pfa_padded_shape(int C, PfaShape &sh) {
+    static const int kBase[6][5] = {{2, 4, 8, 16, 0}, {3, 9, 0, 0, 0},  {5, 0, 0, 0, 0},
+                                    {7, 0, 0, 0, 0},  {11, 0, 0, 0, 0}, {13, 17, 0, 0, 0}};
+    static const std::map<int, int> kOps = {{2, 4},    {3, 16},   {4, 16},  {5, 40},
+                                            {7, 84},   {8, 56},   {9, 120}, {11, 220},
+                                            {13, 312}, {16, 170}, {17, 544}};
+    constexpr double kPass = 12.0;
+    double best = 1e300;
+    int pick[6] = {0, 0, 0, 0, 0, 0}, chosen[6];
+    // every choice of one power (or none) per base; 13 and 17 exclude one
+    // another, which keeps the count small
+    std::function<void(int, long, int, double)> walk = [&](int i, long n, int nf, double per) {
+      if (n > 65535) return;
+      if (i == 6) {
+        if (n < 2L * C - 1 || nf == 0 || per * (double)n >= best) return;
+        best = per * (double)n;
+        std::copy(pick, pick + 6, chosen);
+        return;
+      }
+      pick[i] = 0;
+      walk(i + 1, n, nf, per);
+      for (int q = 0; q < 5 && kBase[i][q] && nf < kPfaMaxFactors; ++q) {
+        pick[i] = kBase[i][q];
+        walk(i + 1, n * pick[i], nf + 1, per + kPass + (double)kOps.at(pick[i]) / pick[i]);
+      }
+      pick[i] = 0;
+    };
+    walk(0, 1, 0, 0.0);
+    if (best == 1e300) return false;
+    sh = PfaShape{};
+    sh.N = 1;
+    for (int q : chosen)
+      if (q) {
+        sh.f[sh.nf++] = q;
+        sh.N *= q;
+      }
+    pfa_strides(sh);
     return true;
   }
 
@@ -312,73 +369,149 @@ class Engine {
     }
   }
 
-  void build_wavelet_fast(const std::vector<WaveletJob<R>> &wj,
-                          const std::vector<long> &wt_base) {
+  // Transform shape of every window, and the largest factor and length.
+  // False when some window has none that fits in shared memory (traces of
+  // over about 14,000 samples, 7,000 in double): the generic kernel serves
+  // all of them then.  wav_padded: some trace length is not itself a
+  // product of supported factors.
+  bool pick_wavelet_shapes(std::vector<PfaShape> &shapes, int &fmax, int &n_max) {
     const char *env = std::getenv("AGD_GPU_GENERIC");
-    if (env != nullptr && env[0] == '1') return;
+    if (env != nullptr && env[0] == '1') return false;
+    std::map<int, PfaShape> by_c;
+    fmax = n_max = 1;
+    wav_padded = false;
+    for (const WindowPlan &W : plan.windows) {
+      auto it = by_c.find(W.C);
+      if (it == by_c.end()) {
+        PfaShape sh;
+        if (!pfa_shape(W.C, sh) && !pfa_padded_shape(W.C, sh)) return false;
+        it = by_c.emplace(W.C, sh).first;
+      }
+      const PfaShape &sh = it->second;
+      if (sh.N != W.C) wav_padded = true;
+      for (int i = 0; i < sh.nf; ++i) fmax = std::max(fmax, sh.f[i]);
+      n_max = std::max(n_max, sh.N);
+      shapes.push_back(sh);
+    }
+    return (size_t)n_max * sizeof(C) <= (size_t)smem_max;
+  }
+
+  // Spectra of the wavelet sources: the plan's where the transform has the
+  // trace's length (and for the generic kernel), the padded ones made on the
+  // device from it where it is longer.
+  void upload_spectra(const std::vector<PfaShape> &shapes) {
+    std::map<int, int> n_of;  // trace length -> transform length
+    for (size_t w = 0; w < shapes.size(); ++w) n_of[plan.windows[w].C] = shapes[w].N;
+    std::vector<C> sp;
+    std::vector<long> so;
+    long c_max = 0;
+    auto length = [&](size_t i) {
+      const auto it = n_of.find(plan.wavelet_n[i]);
+      return it == n_of.end() ? plan.wavelet_n[i] : it->second;
+    };
+    for (size_t i = 0; i < plan.spectra.size(); ++i) {
+      so.push_back((long)sp.size());
+      if (length(i) != plan.wavelet_n[i]) {
+        sp.resize(sp.size() + length(i) / 2 + 1);
+        c_max = std::max(c_max, (long)plan.wavelet_n[i]);
+        continue;
+      }
+      for (const auto &v : plan.spectra[i]) {
+        C c;
+        c.x = (R)v.real();
+        c.y = (R)v.imag();
+        sp.push_back(c);
+      }
+    }
+    spectra.upload(sp, stream);
+    spec_off.upload(so, stream);
+    if (c_max == 0) return;
+    DevArray<double2> half;
+    DevArray<double> taps;
+    half.alloc(c_max / 2 + 1);
+    taps.alloc(c_max);
+    for (size_t i = 0; i < plan.spectra.size(); ++i) {
+      const int n = plan.wavelet_n[i], N = length(i);
+      if (N == n) continue;
+      CK(cudaMemcpyAsync(half.get(), plan.spectra[i].data(),
+                         plan.spectra[i].size() * sizeof(double2), cudaMemcpyHostToDevice,
+                         stream));
+      wavelet_taps<<<n, kWavThreads, 0, stream>>>(half.get(), n, taps.get());
+      wavelet_pad_spectrum<R><<<N / 2 + 1, kWavThreads, 0, stream>>>(taps.get(), n, N,
+                                                                    spectra.get() + so[i]);
+      CK(cudaGetLastError());
+    }
+    CK(cudaStreamSynchronize(stream));  // before the work arrays are released
+  }
+
+  struct WaveletCand {
+    WaveletFn fn;
+    int np;
+  };
+  template <bool PAD, typename Pairs>
+  static void wavelet_candidates(std::vector<WaveletCand> &cands, int fmax, const Pairs &pairs) {
+    if (fmax <= 17) {
+      if constexpr (sizeof(R) == sizeof(float)) {
+        cands.push_back({wavelet_fast<R, 2, 17, PAD>, pairs(80000)});
+        cands.push_back({wavelet_fast<R, 3, 17, PAD>, pairs(60000)});
+        cands.push_back({wavelet_fast<R, 3, 17, PAD>, pairs(40000)});
+        cands.push_back({wavelet_fast<R, 4, 17, PAD>, pairs(40000)});
+      } else {
+        cands.push_back({wavelet_fast<R, 1, 17, PAD>, pairs(80000)});
+        cands.push_back({wavelet_fast<R, 2, 17, PAD>, pairs(80000)});
+      }
+    } else {
+      if constexpr (sizeof(R) == sizeof(float)) {
+        cands.push_back({wavelet_fast<R, 2, 32, PAD>, pairs(60000)});
+        cands.push_back({wavelet_fast<R, 3, 32, PAD>, pairs(60000)});
+        cands.push_back({wavelet_fast<R, 3, 32, PAD>, pairs(40000)});
+      } else {
+        cands.push_back({wavelet_fast<R, 1, 32, PAD>, pairs(60000)});
+      }
+    }
+  }
+
+  void build_wavelet_fast(const std::vector<WaveletJob<R>> &wj,
+                          const std::vector<long> &wt_base,
+                          const std::vector<PfaShape> &shapes, int fmax, int n_max) {
     const int nw = (int)plan.windows.size();
     std::vector<WaveletFastJob<R>> jobs(nw);
     std::vector<unsigned short> perm;
     std::map<int, long> perm_off;
-    int fmax = 1;  // largest factor of any trace length
-    int n_max = 1;
     for (int w = 0; w < nw; ++w) {
-      WaveletFastJob<R> &j = jobs[w];
-      const int N = plan.windows[w].C;
-      if (!pfa_shape(N, j.sh)) return;
-      for (int i = 0; i < j.sh.nf; ++i) fmax = std::max(fmax, j.sh.f[i]);
-      if (!perm_off.count(N)) {
-        perm_off[N] = (long)perm.size();
-        pfa_tables(j.sh, perm);
-      }
-      n_max = std::max(n_max, N);
+      const int N = shapes[w].N;
+      if (perm_off.count(N)) continue;
+      perm_off[N] = (long)perm.size();
+      pfa_tables(shapes[w], perm);
     }
     const size_t per_pair = (size_t)n_max * sizeof(C);
-    if (per_pair > (size_t)smem_max) return;
     pfa_map.upload(perm, stream);
     for (int w = 0; w < nw; ++w) {
       const WindowPlan &W = plan.windows[w];
       WaveletFastJob<R> &j = jobs[w];
+      j.sh = shapes[w];
       j.y = wj[w].y;
       j.src = wj[w].src;
-      j.qmap = pfa_map.get() + perm_off[W.C];
-      j.kpos = j.qmap + W.C;
+      j.qmap = pfa_map.get() + perm_off[j.sh.N];
+      j.kpos = j.qmap + j.sh.N;
       j.blend_rec = blend_rec.get() + wt_base[w];
       j.blend_ts = blend_ts.get() + wt_base[w];
       j.blend_n = blend_n.get() + wt_base[w];
       j.n_traces = W.n_traces;
+      j.C = W.C;
     }
     wavf_jobs.upload(jobs, stream);
     upload_twiddles();
     // candidates: blocks per SM and pairs per block (about a third of the
     // SM's shared memory per block at three blocks)
-    struct Cand {
-      WaveletFn fn;
-      int np;
-    };
-    std::vector<Cand> cands;
+    std::vector<WaveletCand> cands;
     auto pairs = [&](size_t budget) {
       return (int)std::max<size_t>(1, std::min<size_t>(4, budget / per_pair));
     };
-    if (fmax <= 17) {
-      if constexpr (sizeof(R) == sizeof(float)) {
-        cands.push_back(Cand{wavelet_fast<R, 2, 17>, pairs(80000)});
-        cands.push_back(Cand{wavelet_fast<R, 3, 17>, pairs(60000)});
-        cands.push_back(Cand{wavelet_fast<R, 3, 17>, pairs(40000)});
-        cands.push_back(Cand{wavelet_fast<R, 4, 17>, pairs(40000)});
-      } else {
-        cands.push_back(Cand{wavelet_fast<R, 1, 17>, pairs(80000)});
-        cands.push_back(Cand{wavelet_fast<R, 2, 17>, pairs(80000)});
-      }
-    } else {
-      if constexpr (sizeof(R) == sizeof(float)) {
-        cands.push_back(Cand{wavelet_fast<R, 2, 32>, pairs(60000)});
-        cands.push_back(Cand{wavelet_fast<R, 3, 32>, pairs(60000)});
-        cands.push_back(Cand{wavelet_fast<R, 3, 32>, pairs(40000)});
-      } else {
-        cands.push_back(Cand{wavelet_fast<R, 1, 32>, pairs(60000)});
-      }
-    }
+    if (wav_padded)
+      wavelet_candidates<true>(cands, fmax, pairs);
+    else
+      wavelet_candidates<false>(cands, fmax, pairs);
     auto launch_for = [&](TimeLaunch &L, int np) {
       std::vector<int> cj, cp;
       for (int w = 0; w < nw; ++w)
@@ -397,7 +530,7 @@ class Engine {
     if (force != nullptr && force[0] != '\0') {
       pick = std::max(0, std::min(std::atoi(force), (int)cands.size() - 1));
     } else if (cands.size() > 1) {
-      pick = autotune_wavelet(cands.size(), [&](size_t v, TimeLaunch &L) {
+      pick = autotune_wavelet(cands.size(), n_max, [&](size_t v, TimeLaunch &L) {
         launch_for(L, cands[v].np);
         return cands[v].fn;
       });
@@ -414,17 +547,13 @@ class Engine {
   // Times the wavelet candidates (both directions, three rounds, CUDA
   // events), cached per device, precision, trace length and size class.
   template <typename Make>
-  int autotune_wavelet(size_t n, Make make) {
+  int autotune_wavelet(size_t n, int n_max, Make make) {
     long traces = 0;
-    int c_max = 0;
-    for (const WindowPlan &W : plan.windows) {
-      traces += W.n_traces;
-      c_max = std::max(c_max, W.C);
-    }
+    for (const WindowPlan &W : plan.windows) traces += W.n_traces;
     int dev = 0;
     CK(cudaGetDevice(&dev));
     char key[96];
-    std::snprintf(key, sizeof key, "wav:%d:%d:%d:%d", dev, (int)sizeof(R), c_max,
+    std::snprintf(key, sizeof key, "wav%d:%d:%d:%d:%d", wav_padded ? 1 : 0, dev, (int)sizeof(R), n_max,
                   (int)std::log2((double)std::max(1L, traces)));
     static std::mutex mu;
     static std::map<std::string, int> cache;
@@ -1527,21 +1656,12 @@ class Engine {
     if (wavelets) {
       wav_jobs.upload(wj, stream);
       make_time_launch(wav, 2 * (size_t)C_max * sizeof(C), 8, false);
-      // spectra table
-      std::vector<C> sp;
-      std::vector<long> so;
-      for (const auto &s : plan.spectra) {
-        so.push_back((long)sp.size());
-        for (const auto &v : s) {
-          C c;
-          c.x = (R)v.real();
-          c.y = (R)v.imag();
-          sp.push_back(c);
-        }
-      }
-      spectra.upload(sp, stream);
-      spec_off.upload(so, stream);
-      build_wavelet_fast(wj, wt_base);
+      std::vector<PfaShape> shapes;
+      int fmax = 1, n_max = 1;
+      const bool fast = pick_wavelet_shapes(shapes, fmax, n_max);
+      if (!fast) shapes.clear();
+      upload_spectra(shapes);
+      if (fast) build_wavelet_fast(wj, wt_base, shapes, fmax, n_max);
     }
 
     setup_mark("classes");

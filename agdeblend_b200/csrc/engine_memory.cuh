@@ -14,6 +14,7 @@
 #include <mutex>
 #include <memory>
 #include <chrono>
+#include <functional>
 #include <stdexcept>
 #include <string>
 #include <type_traits>

@@ -1,6 +1,8 @@
 // Wavelet convolution / correlation of window traces (reference
-// src/wavelet.c:239-301) for trace lengths C that split into pairwise
-// coprime prime powers of at most 32 (e.g. 2431 = 11 * 13 * 17).
+// src/wavelet.c:239-301) by a transform of length N that splits into
+// pairwise coprime prime powers of at most 32: the trace length C itself
+// where it does (e.g. 2431 = 11 * 13 * 17), else a longer N >= 2 C - 1 (see
+// "Other trace lengths" below).
 //
 // Per trace the reference computes y <- c2r(r2c(y) * S) with S the
 // 1/C-scaled phase spectrum (conjugated for the adjoint), or the bare
@@ -21,9 +23,20 @@
 //  * between them, with Z' the product spectrum,
 //      Z'_k = ((Z_k + conj Z_{C-k}) S_a + (Z_k - conj Z_{C-k}) S_b) / 2,
 //    which is Z_k S when both traces use the same spectrum.  The real and
-//    imaginary parts of the inverse are the two filtered traces.  Traces
-//    without a spectrum use 1/C and are scaled by C when stored, which keeps
-//    the two halves of a pair at the same scale.
+//    imaginary parts of the inverse are the two filtered traces.  A trace
+//    without a spectrum (bare transform pair, i.e. C times the trace) stays
+//    out of the transform, as zeros, and is scaled when the pair is stored:
+//    C times the rounding of its partner would swamp it.
+//
+// Other trace lengths.  The operator is a circular convolution of length C
+// with the real sequence g = c2r(S), so for a C with a large prime (1791 =
+// 9 * 199) the trace is zero-padded to the N >= 2 C - 1 of least arithmetic,
+// multiplied by the length-N spectrum of the zero-padded g, and sample
+// t + C of the linear convolution (t + N - C of the correlation) is added
+// back to sample t.  The cost is that of a transform of twice the length;
+// a length-C transform would need a direct DFT of its prime factor (199
+// products per sample).  13,230 traces of 1791 samples, both directions:
+// 59.8 ms with the direct factor-199 passes, 0.54 ms padded to N = 3696
 //
 // The adjoint reads its traces straight from the blended record (the blend
 // adjoint gather of src/blend.c:1262-1292), so the traces are not written
@@ -39,7 +52,7 @@ constexpr int kPfaMaxFactors = 4;
 constexpr int kWavThreads = 256;
 
 struct PfaShape {
-  int N;                          // transform length C
+  int N;                          // transform length
   int nf;                         // number of factors (axes)
   int f[kPfaMaxFactors];          // pairwise coprime prime powers, outermost axis first
   int g[kPfaMaxFactors];          // dense stride of each axis (product of the later f)
@@ -51,13 +64,13 @@ template <typename R>
 struct WaveletFastJob {
   R *y;                        // window traces [n_traces][C]
   const int *src;              // per trace spectrum index, or -1 (transform pair only)
-  const unsigned short *qmap;  // [C] dense position of sample t
-  const unsigned short *kpos;  // [C] dense position of frequency k after the forward passes
+  const unsigned short *qmap;  // [N] dense position of sample t
+  const unsigned short *kpos;  // [N] dense position of frequency k after the forward passes
   const long *blend_rec;       // per trace: flat record start, or -1 (adjoint gather)
   const int *blend_ts;         // per trace: first blended sample
   const int *blend_n;          // per trace: number of blended samples
   int n_traces;
-  int pad;
+  int C;                       // trace length: N, or at most (N + 1) / 2
   PfaShape sh;
 };
 
@@ -123,18 +136,24 @@ __device__ void pfa_pass_any(int F, Cx<R> *buf, int np, int N, int g, float inv_
 }
 
 // Spectrum value for frequency k of a real signal's length-N transform,
-// conjugated for the adjoint.  A trace without a spectrum (bare transform
-// pair, i.e. N times the trace) gets 1/N here and N when it is stored, so
-// that both traces of a pair keep the same scale through the inverse
-// transform (a factor N between them would cost the smaller one about
-// log10(N) digits).
+// conjugated for the adjoint.
 template <typename R>
 __device__ __forceinline__ Cx<R> spectrum_at(const Cx<R> *sp, int k, int N, bool adjoint) {
   using C = Cx<R>;
-  if (sp == nullptr) return cmake<C>((R)1 / (R)N, (R)0);
   C w = k <= N / 2 ? sp[k] : cmake<C>(sp[N - k].x, -sp[N - k].y);
   if (adjoint) w.y = -w.y;
   return w;
+}
+
+// Input sample t of trace tr: from the record through its blend coordinates
+// (adjoint), or from the traces themselves.
+template <typename R>
+__device__ __forceinline__ R wavelet_input(const WaveletFastJob<R> &job, const R *record, int tr,
+                                           int t) {
+  if (record == nullptr) return job.y[(long)tr * job.C + t];
+  const long r0 = job.blend_rec[tr];
+  const int s0 = job.blend_ts[tr];
+  return r0 >= 0 && t >= s0 && t < s0 + job.blend_n[tr] ? record[r0 + (t - s0)] : (R)0;
 }
 
 // Each CTA transforms np_max pairs of traces of one window (fewer in the
@@ -142,7 +161,8 @@ __device__ __forceinline__ Cx<R> spectrum_at(const Cx<R> *sp, int k, int N, bool
 // -1: correlation of the traces gathered from `record`, written to y.
 // MINB blocks per SM (the register budget of the largest DFT decides which
 // is faster; the engine times the candidates); factors up to FMAX.
-template <typename R, int MINB, int FMAX>
+// PADDED: some window's transform is longer than its traces.
+template <typename R, int MINB, int FMAX, bool PADDED>
 __global__ void __launch_bounds__(kWavThreads, MINB)
     wavelet_fast(const WaveletFastJob<R> *__restrict__ jobs, const int *__restrict__ cta_job,
                  const int *__restrict__ cta_pair0, int np_max,
@@ -154,6 +174,7 @@ __global__ void __launch_bounds__(kWavThreads, MINB)
   const WaveletFastJob<R> &job = jobs[cta_job[blockIdx.x]];
   const PfaShape &sh = job.sh;  // read per pass (a local copy would sit in local memory)
   const int N = sh.N;
+  const int Ct = PADDED ? job.C : N;
   const int n_tr = job.n_traces;
   const int pair0 = cta_pair0[blockIdx.x];
   const int np = min(np_max, ((n_tr + 1) >> 1) - pair0);
@@ -169,19 +190,21 @@ __global__ void __launch_bounds__(kWavThreads, MINB)
     const int tb = ta + 1 < n_tr ? ta + 1 : -1;
     const int mine = tb >= 0 ? ta + (threadIdx.x & 1) : ta;  // this thread's trace
     R *b = reinterpret_cast<R *>(buf + pr * N) + (threadIdx.x & 1);
-    const bool live = tb >= 0 || (threadIdx.x & 1) == 0;
+    const bool live = (tb >= 0 || (threadIdx.x & 1) == 0) && job.src[mine] >= 0;
     if (record != nullptr) {
       const long r0 = job.blend_rec[mine];
       const int s0 = job.blend_ts[mine];
       const int n0 = live && r0 >= 0 ? job.blend_n[mine] : 0;
       for (int t = threadIdx.x >> 1; t < N; t += kWavThreads / 2) {
-        const bool v = t >= s0 && t < s0 + n0;
+        const bool v = t >= s0 && t < s0 + n0;  // a span ends within the trace
         cp_async<sizeof(R)>(b + 2 * __ldg(qmap + t), v ? record + r0 + (t - s0) : record, v);
       }
     } else {
-      const R *y0 = job.y + (long)mine * N;
-      for (int t = threadIdx.x >> 1; t < N; t += kWavThreads / 2)
-        cp_async<sizeof(R)>(b + 2 * __ldg(qmap + t), y0 + t, live);
+      const R *y0 = job.y + (long)mine * Ct;
+      for (int t = threadIdx.x >> 1; t < N; t += kWavThreads / 2) {
+        const bool v = live && (!PADDED || t < Ct);
+        cp_async<sizeof(R)>(b + 2 * __ldg(qmap + t), v ? y0 + t : y0, v);
+      }
     }
   }
   cp_async_commit();
@@ -198,10 +221,14 @@ __global__ void __launch_bounds__(kWavThreads, MINB)
   const int half = N / 2 + 1;
   for (int pr = 0; pr < np; ++pr) {
     const int ta = 2 * (pair0 + pr);
-    const int wa = job.src[ta];
-    const int wb = ta + 1 < n_tr ? job.src[ta + 1] : wa;
-    const C *spa = wa >= 0 ? spectra + spec_off[wa] : nullptr;
-    const C *spb = wb >= 0 ? spectra + spec_off[wb] : nullptr;
+    // a half without a spectrum holds zeros: any spectrum serves it
+    const int sa = job.src[ta];
+    const int sb = ta + 1 < n_tr ? job.src[ta + 1] : sa;
+    const int wa = sa >= 0 ? sa : sb;
+    const int wb = sb >= 0 ? sb : sa;
+    if (wa < 0) continue;
+    const C *spa = spectra + spec_off[wa];
+    const C *spb = spectra + spec_off[wb];
     C *b = buf + pr * N;
     for (int k = threadIdx.x; k < half; k += kWavThreads) {
       const int p = __ldg(kpos + k);
@@ -231,20 +258,74 @@ __global__ void __launch_bounds__(kWavThreads, MINB)
     __syncthreads();
   }
 
-  // ---- store both traces of each pair
+  // ---- store both traces of each pair; a padded transform's samples past
+  // the trace end wrap onto sample t
+  [[maybe_unused]] const int wrap = adjoint ? N - Ct : Ct;
+  [[maybe_unused]] const int w_lo = adjoint ? 1 : 0;  // samples [w_lo, w_hi) take one
+  [[maybe_unused]] const int w_hi = adjoint ? Ct : Ct - 1;
   for (int pr = 0; pr < np; ++pr) {
     const int ta = 2 * (pair0 + pr);
     const bool has_b = ta + 1 < n_tr;
-    R *ya = job.y + (long)ta * N;
+    R *ya = job.y + (long)ta * Ct;
     const C *b = buf + pr * N;
-    const R ka = job.src[ta] < 0 ? (R)N : (R)1;
-    const R kb = has_b && job.src[ta + 1] < 0 ? (R)N : (R)1;
-    for (int t = threadIdx.x; t < N; t += kWavThreads) {
-      const C v = b[__ldg(qmap + t)];
-      ya[t] = v.x * ka;
-      if (has_b) ya[N + t] = v.y * kb;
+    const bool live_a = job.src[ta] >= 0;
+    const bool live_b = has_b && job.src[ta + 1] >= 0;
+    for (int t = threadIdx.x; t < Ct; t += kWavThreads) {
+      C v = b[__ldg(qmap + t)];
+      if constexpr (PADDED) {
+        if (N != Ct && t >= w_lo && t < w_hi) v = cadd(v, b[__ldg(qmap + t + wrap)]);
+      }
+      if (live_a) ya[t] = v.x;
+      if (live_b) ya[Ct + t] = v.y;
+    }
+    for (int h = 0; h < 2; ++h) {  // halves without a spectrum
+      if (h == 0 ? live_a : (live_b || !has_b)) continue;
+      for (int t = threadIdx.x; t < Ct; t += kWavThreads)
+        ya[h * Ct + t] = wavelet_input<R>(job, record, ta + h, t) * (R)Ct;
     }
   }
+}
+
+// ------------------------------------------------- padded spectra (set-up)
+
+// Taps g of the circular convolution whose 1/C-scaled length-C half spectrum
+// is sp (c2r: the imaginary parts of the zero and Nyquist bins are ignored):
+// g[n] = sum_k S_k e^{+2 pi i n k / C} over all k, in double precision.  One
+// block per tap.
+__global__ void __launch_bounds__(kWavThreads)
+    wavelet_taps(const double2 *__restrict__ sp, int C, double *__restrict__ g) {
+  __shared__ double red[32];
+  const long n = blockIdx.x;
+  double acc = 0.0;
+  for (int k = threadIdx.x; k <= C / 2; k += kWavThreads) {
+    double s, c;
+    sincospi(2.0 * (double)((n * k) % C) / (double)C, &s, &c);
+    if (k == 0 || 2 * k == C)
+      acc += sp[k].x * c;
+    else
+      acc += 2.0 * (sp[k].x * c - sp[k].y * s);
+  }
+  const double t = block_sum(acc, red);
+  if (threadIdx.x == 0) g[n] = t;
+}
+
+// Half spectrum of the taps zero-padded to length N, scaled by 1/N:
+// out[k] = (1/N) sum_{n<C} g[n] e^{-2 pi i n k / N}.  One block per bin.
+template <typename R>
+__global__ void __launch_bounds__(kWavThreads)
+    wavelet_pad_spectrum(const double *__restrict__ g, int C, int N, Cx<R> *__restrict__ out) {
+  __shared__ double red_c[32], red_s[32];
+  const long k = blockIdx.x;
+  double re = 0.0, im = 0.0;
+  for (int n = threadIdx.x; n < C; n += kWavThreads) {
+    double s, c;
+    sincospi(2.0 * (double)((n * k) % N) / (double)N, &s, &c);
+    re += g[n] * c;
+    im -= g[n] * s;
+  }
+  const double tr = block_sum(re, red_c);
+  const double ti = block_sum(im, red_s);
+  if (threadIdx.x == 0) out[k] = cmake<Cx<R>>((R)(tr / N), (R)(ti / N));
 }
 
 }  // namespace agd

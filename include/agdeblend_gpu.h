@@ -45,7 +45,8 @@ void agd_gpu_problem_destroy(agd_gpu_problem *problem);
  * spans, [6] device bytes held, [7] blend contributions per forward,
  * [8] 1 if the shape-specialised kernels serve every window, 2 if they
  * serve some, 0 if none, [9] 1 if the prime-factor wavelet kernel serves
- * the problem, [10] and [11] the space-kernel candidates picked by the
+ * the problem with transforms of the traces' own lengths (0: some are
+ * zero-padded to a length it has, or the generic kernel serves them), [10] and [11] the space-kernel candidates picked by the
  * set-up timing for the forward and adjoint of the first window class (-1
  * without shape-specialised kernels), [12] and [13] that class's number of
  * candidates, [14] kernels launched per iteration, [15] window classes on

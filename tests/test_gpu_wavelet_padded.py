@@ -1,0 +1,74 @@
+"""Wavelet stage for trace lengths C with a prime factor above 32
+(agdeblend_b200/csrc/wavelet_fast.cuh): the trace is zero-padded to a
+transform length N >= 2 C - 1 and the wrapped samples are added back.
+Against the float64 oracle at the edges: the smallest lengths, primes, the
+length 1791 = 9 * 199 of a 1500-sample vibroseis trace, odd trace counts,
+pairs with different spectra or none, and a survey that mixes lengths with
+and without padding.  Tolerances are the operator gates of the other wavelet
+tests (1e-5 relative L2 in float, 1e-11 in double)."""
+import numpy as np
+import pytest
+
+import agd_oracle as O
+import agdeblend_b200 as A
+from agdeblend_b200 import synthetic as S
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _survey(specs, seed):
+    """One 2-D patch per (shots, samples, time window, wavelet length), each
+    its own volume with two wavelets; some bad and missing traces."""
+    rng = np.random.default_rng(seed)
+    sv = dict(volumes=[], n_dims=[], window_shapes=[], coords=[], shapes=[], shottimes=[],
+              channels=[], trace_types=[], wavelet_lengths=[], wavelet_idxs=[], wavelets=[])
+    for v, (shots, nt, wt, wl) in enumerate(specs):
+        sv["volumes"].append(v)
+        sv["n_dims"].append(2)
+        sv["window_shapes"].append([shots, wt])
+        sv["coords"].append([0])
+        sv["shapes"].append([shots, nt])
+        sv["shottimes"].append(np.sort(rng.integers(0, shots * nt // 2, shots)).astype(np.int64))
+        sv["channels"].append(np.zeros(shots, np.int32))
+        tt = rng.choice([S.LIVE] * 6 + [S.BAD, S.MISSING], shots).astype(np.int32)
+        tt[0] = S.LIVE
+        sv["trace_types"].append(tt)
+        sv["wavelet_lengths"] += [wl, wl]
+        sv["wavelets"] += [rng.standard_normal(wl).astype(np.float32) for _ in range(2)]
+        sv["wavelet_idxs"].append((2 * v + rng.integers(0, 2, shots)).astype(np.int32))
+    return sv
+
+
+CASES = {
+    "C31": [(9, 22, 8, 4)],
+    "C37": [(8, 20, 16, 6)],
+    "C997": [(5, 930, 64, 38)],
+    "C1791": [(7, 1500, 256, 256)],
+    "C2431_and_1791": [(6, 2048, 256, 256), (5, 1500, 256, 256)],
+}
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_padded_wavelet_vs_oracle(name, dtype):
+    tol = 1e-5 if dtype == np.float32 else 1e-11
+    sv = _survey(CASES[name], seed=len(name))
+    plan = O.make_plan(**sv)
+    if name.startswith("C") and "_" not in name:
+        assert {w.conv for w in plan.windows} == {int(name[1:])}
+    prob = A.Problem(dtype=dtype, **sv)
+    assert prob.info[9] == 0 and prob.kernels()["wavelet"] == "wavelet_fast"
+    rec = np.random.default_rng(1).standard_normal(prob.record_size)
+    O.apply_mute(plan.cfg, rec)
+    x = O.model_to_flat(O.adjoint(plan, rec))
+    x_ref = np.stack([x.real, x.imag], -1).reshape(-1)
+    assert rel_l2(prob.adjoint(rec), x_ref) <= tol
+    y_ref = O.forward(plan, O.flat_to_model(plan, x))
+    assert rel_l2(prob.forward(x_ref), y_ref) <= tol
+    for p, (o, r) in enumerate(zip(prob.set_output(x_ref),
+                                   O.set_output(plan, O.flat_to_model(plan, x)))):
+        # traces without a spectrum carry a factor C (the bare transform pair)
+        scale = np.where(sv["trace_types"][p] == S.LIVE, 1.0, 1.0 / plan.conv[p])[:, None]
+        assert rel_l2(o * scale, r * scale) <= tol
+    prob.close()
