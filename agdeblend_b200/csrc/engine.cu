@@ -184,7 +184,8 @@ int agd_gpu_problem_info(agd_gpu_problem const *pb, long int *info) {
   info[20] = e.wav_fast ? e.wav_pick : -1;
   info[21] = e.wav_candidates;
   long n_line = 0;
-  for (char c : e.win_line) n_line += c ? 1 : 0;
+  for (size_t w = 0; w < e.win_dft.size(); ++w)
+    n_line += e.win_dft[w] && e.plan.windows[w].D == 1 ? 1 : 0;
   info[22] = n_line;
   return 0;
 }
@@ -193,10 +194,13 @@ int agd_gpu_problem_kernels(agd_gpu_problem const *pb, char *buf, int len) {
   if (pb == nullptr || buf == nullptr || len <= 0) return 1;
   const agd::EngineR &e = *pb->eng;
   const bool sc = !e.classes.empty(), tg = !e.tgroups.empty();
+  const char *other = e.dft_fwd[0].b.n   ? "plane_dft"  // without window classes
+                      : e.dft_fwd[1].b.n ? "line_dft"
+                                         : "axis_pass";
   const int n = std::snprintf(
       buf, (size_t)len, "space_fwd=%s space_adj=%s time_fwd=%s time_adj=%s wavelet=%s",
-      !sc ? "axis_pass" : (e.classes[0]->tc ? "space_fwd_tc" : e.classes[0]->fv().name),
-      !sc ? "axis_pass" : (e.classes[0]->tc ? "space_adj_tc" : e.classes[0]->av().name),
+      !sc ? other : (e.classes[0]->tc ? "space_fwd_tc" : e.classes[0]->fv().name),
+      !sc ? other : (e.classes[0]->tc ? "space_adj_tc" : e.classes[0]->av().name),
       tg ? e.tgroups[0]->fv().name : "time_c2r_ola", tg ? e.tgroups[0]->av().name : "time_r2c",
       !e.wavelets ? "none" : (e.wav_fast ? "wavelet_fast" : "wavelet_apply"));
   return n < 0 || n >= len ? 1 : 0;
@@ -237,7 +241,7 @@ int agd_gpu_adjoint(agd_gpu_problem *pb, AGD_TYPE const *record, AGD_TYPE *model
     for (const auto &cp : e.classes) e.launch_space_adj(*cp, cp->pl_adj_plain, agd::kStore, 0, 0);
     for (size_t k = 0; k < e.adj_plain.size(); ++k)
       e.launch_axis(e.adj_plain[k], 0, agd::kStore, 0, 0);
-    e.launch_line_adj(e.line_adj_plain, agd::kStore, 0, 0);
+    e.launch_dft_adj(e.dft_adj_plain, agd::kStore, 0, 0);
     e.model_to_ref(e.G.get(), model);
     e.check_tc_error();
     return 0;

@@ -62,19 +62,30 @@ class Engine {
   DevArray<double> dscalar;
 
   std::vector<AxisLaunch> fwd, adj_update, adj_plain;
-  // windows with one space axis of a length without a shape-specialised
-  // kernel, on the line kernels (line_dft.cuh)
-  struct LineLaunch {
-    DevArray<LineJob<R>> jobs;
-    DevArray<int> cta_job;
-    DevArray<long> cta_line0;
-    int n_cta = 0;
+  // windows without a shape-specialised space kernel, on the table-DFT
+  // kernels (plane_dft.cuh): the last one or two axes, then one pass per
+  // further axis (forward; the adjoint in the other order)
+  struct DftBatches {
+    DevArray<int> job;
+    DevArray<long> first;
+    int n = 0, grid = 0;
     size_t smem = 0;
   };
-  LineLaunch line_fwd, line_adj, line_adj_plain;
-  DevArray<R> line_tab;        // per (P, L): forward and adjoint cos / sin tables
-  std::vector<char> win_line;  // 1: window on the line kernels
-  std::vector<LineJob<R>> line_adj_host;  // adjoint jobs (the plain adjoint's, re-aimed)
+  struct PlaneDftLaunch {
+    DevArray<PlaneDftJob<R>> jobs;
+    DftBatches b;
+  };
+  struct AxisDftLaunch {
+    DevArray<AxisDftJob<R>> jobs;
+    DftBatches b;
+  };
+  // planes of two axes ([0]) and lines of one ([1])
+  PlaneDftLaunch dft_fwd[2], dft_adj[2], dft_adj_plain[2];
+  int line_nt = kDftThreads;  // threads of the line kernel's blocks
+  std::vector<AxisDftLaunch> dft_fwd_axes, dft_adj_axes;
+  DevArray<R> dft_tab;        // cos / sin tables of every padded length
+  std::vector<char> win_dft;  // axes in the window's plane kernel (2 or 1), 0: not on these kernels
+  std::vector<PlaneDftJob<R>> dft_adj_host[2];  // adjoint jobs (the plain adjoint's, re-aimed)
   TimeLaunch time_fwd, time_adj, wav;
 
   // Shape-specialised kernels (fast.cuh).  Windows are grouped into classes
@@ -230,7 +241,12 @@ class Engine {
     const int limit = smem_max;
     smem_max = std::min({opt_in(axis_pass<R>, limit), opt_in(time_c2r_ola<R>, limit),
                          opt_in(time_r2c<R>, limit), opt_in(wavelet_apply<R>, limit),
-                         opt_in(line_dft_fwd<R>, limit), opt_in(line_dft_adj<R>, limit)});
+                         opt_in(plane_dft<R, true>, limit), opt_in(plane_dft<R, false>, limit),
+                         opt_in(axis_dft<R, true>, limit), opt_in(axis_dft<R, false>, limit),
+                         opt_in(line_dft<R, true, 128>, limit),
+                         opt_in(line_dft<R, false, 128>, limit),
+                         opt_in(line_dft<R, true, 256>, limit),
+                         opt_in(line_dft<R, false, 256>, limit)});
     opt_in_wavelet<false>(limit);
     opt_in_wavelet<true>(limit);
   }
@@ -928,144 +944,266 @@ class Engine {
       win_class[w] = k;
       classes[k]->win.push_back(w);
     }
-    // one space axis of any other length up to kLineMaxP: line kernels,
-    // when their blocks fit in shared memory
-    win_line.assign(nw, 0);
+    // any other shape up to kDftMaxP per axis: table-DFT kernels, with the
+    // last two axes in one kernel when a plane of them fits in shared memory
+    win_dft.assign(nw, 0);
     for (int w = 0; w < nw && !generic_only; ++w) {
       const WindowPlan &W = plan.windows[w];
-      if (win_class[w] >= 0 || W.D != 1 || W.P[0] > kLineMaxP || W.P[0] < 3) continue;
-      const int P = W.P[0], L = W.L[0];
-      const int H = (P - 1) / 2;
-      const size_t sf = line_fwd_smem<R>(P, H, (L + 3) / 4 * 4, 4);
-      const size_t sa = line_adj_smem<R>(P, L, (P / 2 + 1 + 3) / 4 * 4, 4);
-      if (std::max(sf, sa) <= (size_t)smem_max) win_line[w] = 1;
+      if (win_class[w] >= 0) continue;
+      bool ok = true, plane = W.D > 1;
+      for (int d = 0; d < W.D; ++d) ok = ok && W.P[d] >= 3 && W.P[d] <= kDftMaxP;
+      if (!ok) continue;
+      for (bool fwd : {true, false}) {
+        const DftAxis<R> b = dft_axis(W, W.D - 1, fwd);
+        ok = ok && line_dft_smem<R>(b, 4) <= (size_t)smem_max;
+        for (int d = 0; d + 1 < W.D; ++d)
+          ok = ok && axis_dft_smem<R>(dft_axis(W, d, fwd), 32) <= (size_t)smem_max;
+        plane = plane &&
+                plane_dft_smem<R>(dft_axis(W, W.D - 2, fwd), b, 1) <= (size_t)smem_max;
+      }
+      if (ok) win_dft[w] = plane ? 2 : 1;
     }
     n_generic = 0;
     max_d_generic = 0;
     for (int w = 0; w < nw; ++w)
-      if (win_class[w] < 0 && !win_line[w]) {
+      if (win_class[w] < 0 && !win_dft[w]) {
         ++n_generic;
         max_d_generic = std::max(max_d_generic, plan.windows[w].D);
       }
   }
 
-  // Line-kernel jobs, tables and block lists (windows marked in win_line).
-  // Tables per (P, L) in double precision, rounded once: forward rows
-  // j = 1 .. (P-1)/2 over outputs k < L, adjoint rows j < L over k <= P/2,
-  // cos / sin of 2 pi (j k mod P) / P, rows padded to a multiple of 4.
-  void build_line_kernels() {
+  // One axis of a window for the table-DFT kernels (table pointer filled in
+  // by build_dft_kernels).
+  static DftAxis<R> dft_axis(const WindowPlan &W, int d, bool fwd) {
+    DftAxis<R> x{};
+    x.P = W.P[d];
+    x.H = (x.P - 1) / 2;
+    x.kpad = (x.P / 2 + kDftTk<R>) / kDftTk<R> * kDftTk<R>;
+    x.n_in = fwd ? W.P[d] : W.L[d];
+    x.n_out = fwd ? W.L[d] : W.P[d];
+    return x;
+  }
+
+  // Table-DFT jobs, tables and batch lists (windows marked in win_dft).
+  // Tables per padded length P in double precision, rounded once: rows
+  // j = 1 .. (P-1)/2 over outputs k <= P/2, cos then sin of
+  // 2 pi (j k mod P) / P.
+  void build_dft_kernels() {
     const int nw = (int)plan.windows.size();
     std::vector<R> tab;
-    std::map<std::pair<int, int>, std::pair<long, long>> off;  // (P, L) -> fwd, adj
-    auto add_table = [&](int P, int rows, int j0, int kout, int kpad) {
-      const long o = (long)tab.size();
-      tab.resize(tab.size() + 2 * (size_t)rows * kpad, (R)0);
-      for (int r = 0; r < rows; ++r)
-        for (int k = 0; k < kout; ++k) {
-          const long m = (long)(r + j0) * k % P;
-          const double a = 2.0 * 3.14159265358979323846 * (double)m / (double)P;
-          tab[o + (long)r * kpad + k] = (R)std::cos(a);
-          tab[o + (long)rows * kpad + (long)r * kpad + k] = (R)std::sin(a);
-        }
-      return o;
+    std::map<int, long> off;  // P -> table
+    auto axis = [&](const WindowPlan &W, int d, bool fwd) {
+      DftAxis<R> x = dft_axis(W, d, fwd);
+      auto it = off.find(x.P);
+      if (it == off.end()) {
+        const long o = (long)tab.size();
+        tab.resize(tab.size() + dft_table_reals(x), (R)0);
+        for (int r = 0; r < x.H; ++r)
+          for (int k = 0; k <= x.P / 2; ++k) {
+            const long m = (long)(r + 1) * k % x.P;
+            const double t = 2.0 * 3.14159265358979323846 * (double)m / (double)x.P;
+            tab[o + (long)r * x.kpad + k] = (R)std::cos(t);
+            tab[o + ((long)x.H + r) * x.kpad + k] = (R)std::sin(t);
+          }
+        it = off.emplace(x.P, o).first;
+      }
+      // an offset for now; the address once the table is on the device
+      x.tab = reinterpret_cast<const R *>(it->second * (long)sizeof(R));
+      return x;
     };
-    std::vector<LineJob<R>> jf, ja;
-    std::vector<long> tf, ta;  // table offsets of each job
+    C *Sb[2] = {S0.get(), S1.get()};
+    std::vector<PlaneDftJob<R>> jf[2], ja[2];  // planes, lines
+    int n_axes = 0;  // single-axis passes
+    for (int w = 0; w < nw; ++w)
+      if (win_dft[w]) n_axes = std::max(n_axes, plan.windows[w].D - win_dft[w]);
+    std::vector<std::vector<AxisDftJob<R>>> xf(n_axes), xa(n_axes);
     for (int w = 0; w < nw; ++w) {
-      if (!win_line[w]) continue;
+      if (!win_dft[w]) continue;
       const WindowPlan &W = plan.windows[w];
-      const int P = W.P[0], L = W.L[0];
-      const int H = (P - 1) / 2;
-      const int kpf = (L + 3) / 4 * 4, kpa = (P / 2 + 1 + 3) / 4 * 4;
-      auto it = off.find({P, L});
-      if (it == off.end())
-        it = off.emplace(std::make_pair(P, L),
-                         std::make_pair(add_table(P, H, 1, L, kpf),
-                                        add_table(P, L, 0, P / 2 + 1, kpa)))
-                 .first;
-      const long lines = (long)W.T * W.F;
-      LineJob<R> f{};
-      f.src = X.get() + W.model_off;
-      f.dst = S0.get() + W.model_off;
-      f.lines = lines;
-      f.P = P;
-      f.L = L;
-      f.rows = H;
-      f.kout = L;
-      f.kpad = kpf;
+      const bool plane = win_dft[w] == 2;
+      const int extra = W.D - win_dft[w];  // single-axis passes
+      PlaneDftJob<R> f{};
+      f.planes = (long)W.T * W.F;
+      for (int d = 0; d < extra; ++d) f.planes *= W.P[d];
       f.pid = W.problem;
-      LineJob<R> a = f;
-      a.src = S0.get() + W.model_off;
-      a.dst = X.get() + W.model_off;
-      a.rows = L;
-      a.kout = P / 2 + 1;
-      a.kpad = kpa;
-      f.nl = line_pick_nl(P, L, true);
-      a.nl = line_pick_nl(P, L, false);
-      jf.push_back(f);
-      ja.push_back(a);
-      tf.push_back(it->second.first);
-      ta.push_back(it->second.second);
-    }
-    if (jf.empty()) return;
-    line_tab.upload(tab, stream);
-    for (size_t i = 0; i < jf.size(); ++i) {
-      jf[i].tab_c = line_tab.get() + tf[i];
-      jf[i].tab_s = jf[i].tab_c + (long)jf[i].rows * jf[i].kpad;
-      ja[i].tab_c = line_tab.get() + ta[i];
-      ja[i].tab_s = ja[i].tab_c + (long)ja[i].rows * ja[i].kpad;
-    }
-    make_line_launch(line_fwd, jf, true);
-    make_line_launch(line_adj, ja, false);
-    line_adj_host = ja;
-  }
-
-  // Lines per block of a window: a multiple of 4 whose 4-line x 4-output
-  // tiles best fill the block's threads, within a shared-memory budget of
-  // three blocks per SM (two in double; more when even 4 lines need it),
-  // counting the memory the system reserves per block and the kernels'
-  // static arrays (at most 256 bytes).
-  int line_pick_nl(int P, int L, bool fwd) const {
-    const int H = (P - 1) / 2;
-    const int kpad = fwd ? (L + 3) / 4 * 4 : (P / 2 + 1 + 3) / 4 * 4;
-    auto smem = [&](int nl) {
-      return fwd ? line_fwd_smem<R>(P, H, kpad, nl) : line_adj_smem<R>(P, L, kpad, nl);
-    };
-    const int blocks = sizeof(R) == sizeof(float) ? 3 : 2;
-    const size_t budget =
-        std::max<size_t>((size_t)(sm_smem / blocks - block_reserved - 256), smem(4));
-    int best = 4;
-    double best_eff = -1.0;
-    for (int nl = 4; nl <= 64 && smem(nl) <= budget; nl += 4) {
-      const int tiles = nl / 4 * (kpad / 4);
-      const int rounds = (tiles + kLineThreads - 1) / kLineThreads;
-      const double eff = (double)tiles / (rounds * kLineThreads);
-      if (eff >= best_eff - 1e-9) {
-        best_eff = eff;
-        best = nl;
+      PlaneDftJob<R> g = f;
+      if (plane) f.a = axis(W, W.D - 2, true);
+      f.b = axis(W, W.D - 1, true);
+      f.src = X.get() + W.model_off;
+      f.dst = Sb[extra & 1] + W.model_off;
+      if (plane) g.a = axis(W, W.D - 2, false);
+      g.b = axis(W, W.D - 1, false);
+      g.src = Sb[extra & 1] + W.model_off;
+      g.dst = X.get() + W.model_off;
+      jf[plane ? 0 : 1].push_back(f);
+      ja[plane ? 0 : 1].push_back(g);
+      for (int t = 0; t < extra; ++t) {
+        // forward: axis extra-1-t; adjoint: axis t (the time kernels' side
+        // is S0 in both directions)
+        for (bool fwd : {true, false}) {
+          const int d = fwd ? extra - 1 - t : t;
+          AxisDftJob<R> x{};
+          x.outer = (long)W.T * W.F;
+          for (int e = 0; e < d; ++e) x.outer *= W.P[e];
+          x.inner = 1;
+          for (int e = d + 1; e < W.D; ++e) x.inner *= W.L[e];
+          x.a = axis(W, d, fwd);
+          x.src = Sb[(fwd ? extra - t : t) & 1] + W.model_off;
+          x.dst = Sb[(fwd ? extra - t - 1 : t + 1) & 1] + W.model_off;
+          (fwd ? xf : xa)[t].push_back(x);
+        }
       }
     }
-    return best;
+    if (jf[0].empty() && jf[1].empty()) return;
+    dft_tab.upload(tab, stream);
+    auto place = [&](DftAxis<R> &x) {
+      if (x.P > 1) x.tab = dft_tab.get() + reinterpret_cast<uintptr_t>(x.tab) / sizeof(R);
+    };
+    for (auto *v : {&jf[0], &jf[1], &ja[0], &ja[1]})
+      for (auto &j : *v) {
+        place(j.a);
+        place(j.b);
+      }
+    pick_plane_batches(jf[0]);
+    pick_plane_batches(ja[0]);
+    // lines: 256-thread blocks share the tables of long axes
+    int table = 0;
+    for (const auto &j : jf[1]) table = std::max(table, dft_table_reals(j.b));
+    line_nt = table * sizeof(R) > 8192 ? 256 : 128;
+    pick_line_batches(jf[1]);
+    pick_line_batches(ja[1]);
+    for (int k = 0; k < 2; ++k) {
+      make_plane_dft(dft_fwd[k], jf[k], k == 1, plane_kernel(k == 1, true));
+      make_plane_dft(dft_adj[k], ja[k], k == 1, plane_kernel(k == 1, false));
+      dft_adj_host[k] = ja[k];
+    }
+    dft_fwd_axes.resize(n_axes);
+    dft_adj_axes.resize(n_axes);
+    for (int t = 0; t < n_axes; ++t)
+      for (bool fwd : {true, false}) {
+        auto &v = (fwd ? xf : xa)[t];
+        for (auto &j : v) {
+          place(j.a);
+          j.nl = pick_axis_lines(j.a);
+        }
+        if (fwd)
+          make_axis_dft(dft_fwd_axes[t], v, axis_dft<R, true>);
+        else
+          make_axis_dft(dft_adj_axes[t], v, axis_dft<R, false>);
+      }
   }
 
-  void make_line_launch(LineLaunch &Lc, const std::vector<LineJob<R>> &jobs, bool fwd) {
-    std::vector<int> cj;
-    std::vector<long> cl;
+  using PlaneDftFn = void (*)(const PlaneDftJob<R> *, const int *, const long *, int, int, R, R,
+                              const R *, const R *, R *);
+  PlaneDftFn plane_kernel(bool line, bool fwd) const {
+    if (!line) return fwd ? plane_dft<R, true> : plane_dft<R, false>;
+    if (line_nt == 256) return fwd ? line_dft<R, true, 256> : line_dft<R, false, 256>;
+    return fwd ? line_dft<R, true, 128> : line_dft<R, false, 128>;
+  }
+
+  // shared memory of a block of nt threads at the four (float) or three
+  // (double) times 128 threads per SM that the table-DFT kernels are
+  // compiled for
+  size_t dft_budget(int nt) const {
+    const int blocks = (sizeof(R) == sizeof(float) ? 512 : 384) / nt;
+    return (size_t)(sm_smem / blocks - block_reserved);
+  }
+
+  // Warp iterations of the product loop over n_lines lines of one axis.
+  static double dft_warp_work(const DftAxis<R> &x, int n_lines) {
+    const int tiles = (n_lines + 3) / 4 * (x.kpad / kDftTk<R>);
+    return (double)((tiles + 31) / 32) * (x.H + 6);
+  }
+
+  // Planes per batch of every job: the number with the least warp work per
+  // plane (whole warps of 4-line tiles; the constant stands for a batch's
+  // barriers and first loads), within a block's share of the shared memory
+  // and small enough that the batches fill the device.
+  void pick_plane_batches(std::vector<PlaneDftJob<R>> &jobs) const {
+    long total = 0;
+    for (const auto &j : jobs) total += j.planes;
+    const long most = std::min<long>(32, std::max<long>(1, total / (4L * n_sm)));
+    for (auto &j : jobs) {
+      double best = 1e300;
+      j.np = 1;
+      for (int np = 1; np <= most; ++np) {
+        if (np > 1 && plane_dft_smem<R>(j.a, j.b, np) > dft_budget(kDftThreads)) break;
+        const double work = (dft_warp_work(j.a, np * j.b.n_in) +
+                             dft_warp_work(j.b, np * j.a.n_out) + 40.0) / np;
+        if (work < best) {
+          best = work;
+          j.np = np;
+        }
+      }
+    }
+  }
+
+  // Lines per batch of every job of the line kernel: at most one tile per
+  // thread, the block's share of the shared memory, and few enough that the
+  // batches fill the device.
+  void pick_line_batches(std::vector<PlaneDftJob<R>> &jobs) const {
+    long total = 0;
+    for (const auto &j : jobs) total += j.planes;
+    const long cap = std::max<long>(4, total / (512 / line_nt * (long)n_sm) / 4 * 4);
+    for (auto &j : jobs) {
+      long nl = std::min<long>(4L * (line_nt / (j.b.kpad / kDftTk<R>)), cap);
+      while (nl > 4 && line_dft_smem<R>(j.b, nl) > dft_budget(line_nt)) nl -= 4;
+      j.np = (int)std::max<long>(4, nl);
+    }
+  }
+
+  int pick_axis_lines(const DftAxis<R> &x) const {
+    int nl = 32;
+    while (nl < 256 && axis_dft_smem<R>(x, nl + 32) <= dft_budget(kDftThreads)) nl += 32;
+    return nl;
+  }
+
+  template <typename K>
+  void finish_dft_batches(DftBatches &B, const std::vector<int> &job,
+                          const std::vector<long> &first, size_t smem, int nt, K kernel) {
+    B.job.upload(job, stream);
+    B.first.upload(first, stream);
+    B.n = (int)job.size();
+    B.smem = smem;
+    int per_sm = 1;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, nt, smem));
+    B.grid = std::max(1, std::min(B.n, std::max(per_sm, 1) * n_sm));
+  }
+
+  template <typename K>
+  void make_plane_dft(PlaneDftLaunch &L, const std::vector<PlaneDftJob<R>> &jobs, bool line,
+                      K kernel) {
+    if (jobs.empty()) return;
+    std::vector<int> bj;
+    std::vector<long> bp;
     size_t smem = 0;
     for (size_t i = 0; i < jobs.size(); ++i) {
-      const LineJob<R> &j = jobs[i];
-      for (long l = 0; l < j.lines; l += j.nl) {
-        cj.push_back((int)i);
-        cl.push_back(l);
+      for (long p = 0; p < jobs[i].planes; p += jobs[i].np) {
+        bj.push_back((int)i);
+        bp.push_back(p);
       }
-      smem = std::max(smem, fwd ? line_fwd_smem<R>(j.P, j.rows, j.kpad, j.nl)
-                                : line_adj_smem<R>(j.P, j.L, j.kpad, j.nl));
+      smem = std::max(smem, line ? line_dft_smem<R>(jobs[i].b, jobs[i].np)
+                                 : plane_dft_smem<R>(jobs[i].a, jobs[i].b, jobs[i].np));
     }
-    Lc.jobs.upload(jobs, stream);
-    Lc.cta_job.upload(cj, stream);
-    Lc.cta_line0.upload(cl, stream);
-    Lc.n_cta = (int)cj.size();
-    Lc.smem = smem;
+    L.jobs.upload(jobs, stream);
+    finish_dft_batches(L.b, bj, bp, smem, line ? line_nt : kDftThreads, kernel);
+  }
+
+  template <typename K>
+  void make_axis_dft(AxisDftLaunch &L, const std::vector<AxisDftJob<R>> &jobs, K kernel) {
+    std::vector<int> bj;
+    std::vector<long> bl;
+    size_t smem = 0;
+    for (size_t i = 0; i < jobs.size(); ++i) {
+      const long lines = jobs[i].outer * jobs[i].inner;
+      for (long l = 0; l < lines; l += jobs[i].nl) {
+        bj.push_back((int)i);
+        bl.push_back(l);
+      }
+      smem = std::max(smem, axis_dft_smem<R>(jobs[i].a, jobs[i].nl));
+    }
+    L.jobs.upload(jobs, stream);
+    finish_dft_batches(L.b, bj, bl, smem, kDftThreads, kernel);
   }
 
   // Times every candidate of a class (three rounds over the candidates, each
@@ -1595,7 +1733,9 @@ class Engine {
     pick_classes();
     X.alloc_pooled(M);
     S0.alloc_pooled(M);
-    if (n_generic) S1.alloc_pooled(M);
+    bool second = n_generic > 0;  // a second intermediate: generic passes, single-axis passes
+    for (int w = 0; w < nw; ++w) second = second || (win_dft[w] && plan.windows[w].D > win_dft[w]);
+    if (second) S1.alloc_pooled(M);
     Y.alloc_pooled(toff);
     rec_d.alloc_pooled(plan.record_size);
     rec_r.alloc_pooled(plan.record_size);
@@ -1619,7 +1759,7 @@ class Engine {
     for (int w = 0; w < nw; ++w) {
       const WindowPlan &W = plan.windows[w];
       TimeJob<R> &j = tj[w];
-      j.z = (win_class[w] >= 0 ? S0.get() : Sb[(W.D - 1) & 1]) + W.model_off;
+      j.z = (win_class[w] >= 0 || win_dft[w] ? S0.get() : Sb[(W.D - 1) & 1]) + W.model_off;
       j.y = Y.get() + trace_off[w];
       j.space_scale = space_scale.get() + wt_base[w];
       j.time_taper = time_taper.get() + ttaper_off[w];
@@ -1665,8 +1805,8 @@ class Engine {
     }
 
     setup_mark("classes");
-    // ---- one-axis windows of other lengths (line kernels)
-    build_line_kernels();
+    // ---- windows of other shapes (table-DFT kernels)
+    build_dft_kernels();
 
     // ---- space-axis passes (generic path)
     maxD = max_d_generic;
@@ -1677,7 +1817,7 @@ class Engine {
       std::vector<AxisJob<R>> jf, ju, jp;
       for (int w = 0; w < nw; ++w) {
         const WindowPlan &W = plan.windows[w];
-        if (W.D <= k || win_class[w] >= 0 || win_line[w]) continue;
+        if (W.D <= k || win_class[w] >= 0 || win_dft[w]) continue;
         const long TF = (long)W.T * W.F;
         {  // forward: axis D-1-k, inverse FFT, crop P -> L
           const int a = W.D - 1 - k;
@@ -1723,7 +1863,7 @@ class Engine {
       pending_plain.push_back(jp);
     }
 
-    setup_mark("line, generic");
+    setup_mark("dft, generic");
     // ---- forward blend: window traces into the record, window then trace
     {
       std::vector<Contrib> list;
@@ -1806,18 +1946,18 @@ class Engine {
       size_t i = 0;
       for (int w = 0; w < (int)plan.windows.size(); ++w) {
         const WindowPlan &W = plan.windows[w];
-        if (W.D <= (int)k || win_class[w] >= 0 || win_line[w]) continue;
+        if (W.D <= (int)k || win_class[w] >= 0 || win_dft[w]) continue;
         if ((int)k == W.D - 1) jobs[i].dst = G.get() + W.model_off;
         ++i;
       }
       make_axis_launch(adj_plain[k], jobs);
     }
-    if (!line_adj_host.empty()) {
-      std::vector<LineJob<R>> jobs = line_adj_host;
+    for (int k = 0; k < 2; ++k) {
+      std::vector<PlaneDftJob<R>> jobs = dft_adj_host[k];
       size_t i = 0;
       for (int w = 0; w < (int)plan.windows.size(); ++w)
-        if (win_line[w]) jobs[i++].dst = G.get() + plan.windows[w].model_off;
-      make_line_launch(line_adj_plain, jobs, false);
+        if (win_dft[w] == 2 - k) jobs[i++].dst = G.get() + plan.windows[w].model_off;
+      make_plane_dft(dft_adj_plain[k], jobs, k == 1, plane_kernel(k == 1, false));
     }
     CK(cudaStreamSynchronize(stream));
   }
@@ -1918,31 +2058,45 @@ class Engine {
     }
   }
 
-  void launch_line_fwd() {
-    if (line_fwd.n_cta == 0) return;
-    line_dft_fwd<R><<<line_fwd.n_cta, kLineThreads, line_fwd.smem, stream>>>(
-        line_fwd.jobs.get(), line_fwd.cta_job.get(), line_fwd.cta_line0.get());
+  void launch_axis_dft(const AxisDftLaunch &L, bool forward) {
+    if (L.b.n == 0) return;
+    auto fn = forward ? axis_dft<R, true> : axis_dft<R, false>;
+    fn<<<L.b.grid, kDftThreads, L.b.smem, stream>>>(L.jobs.get(), L.b.job.get(), L.b.first.get(),
+                                                    L.b.n);
     CK(cudaGetLastError());
   }
 
-  void launch_line_adj(const LineLaunch &Lc, int epilogue, R step, R lamb,
-                       const R *lamb_dev = nullptr) {
-    if (Lc.n_cta == 0) return;
-    line_dft_adj<R><<<Lc.n_cta, kLineThreads, Lc.smem, stream>>>(
-        Lc.jobs.get(), Lc.cta_job.get(), Lc.cta_line0.get(), epilogue, step, lamb,
+  void launch_plane_dft(const PlaneDftLaunch &L, bool line, bool forward, int epilogue, R step,
+                        R lamb, const R *lamb_dev) {
+    if (L.b.n == 0) return;
+    plane_kernel(line, forward)<<<L.b.grid, line ? line_nt : kDftThreads, L.b.smem, stream>>>(
+        L.jobs.get(), L.b.job.get(), L.b.first.get(), L.b.n, epilogue, step, lamb,
         multi ? step_dev.get() : nullptr, lamb_dev, multi ? pmax.get() : scalar.get());
     CK(cudaGetLastError());
   }
 
+  void launch_dft_fwd() {
+    for (int k = 0; k < 2; ++k)
+      launch_plane_dft(dft_fwd[k], k == 1, true, kStore, (R)0, (R)0, nullptr);
+    for (const auto &x : dft_fwd_axes) launch_axis_dft(x, true);
+  }
+
+  void launch_dft_adj(const PlaneDftLaunch (&L)[2], int epilogue, R step, R lamb,
+                      const R *lamb_dev = nullptr) {
+    for (const auto &x : dft_adj_axes) launch_axis_dft(x, false);
+    for (int k = 0; k < 2; ++k)
+      launch_plane_dft(L[k], k == 1, false, epilogue, step, lamb, lamb_dev);
+  }
+
   void launch_space_fwd_all() {
     for (const auto &cp : classes) launch_space_fwd(*cp);
-    launch_line_fwd();
+    launch_dft_fwd();
     for (size_t k = 0; k < fwd.size(); ++k) launch_axis(fwd[k], 1, kStore, 0, 0);
   }
 
   void launch_space_adj_all(int epilogue, R step, R lamb, const R *lamb_dev) {
     for (const auto &cp : classes) launch_space_adj(*cp, cp->pl_adj, epilogue, step, lamb, lamb_dev);
-    launch_line_adj(line_adj, epilogue, step, lamb, lamb_dev);
+    launch_dft_adj(dft_adj, epilogue, step, lamb, lamb_dev);
     for (size_t k = 0; k < adj_update.size(); ++k)
       launch_axis(adj_update[k], 0, epilogue, step, lamb, lamb_dev);
   }
@@ -2005,7 +2159,8 @@ class Engine {
     for (const auto &gp : tgroups) n += (gp->tf.n_cta ? 1 : 0) + (gp->ta.n_cta ? 1 : 0);
     for (const auto *v : {&fwd, &adj_update})
       for (const AxisLaunch &L : *v) n += L.n_cta ? 1 : 0;
-    n += (line_fwd.n_cta ? 1 : 0) + (line_adj.n_cta ? 1 : 0);
+    for (int k = 0; k < 2; ++k) n += (dft_fwd[k].b.n ? 1 : 0) + (dft_adj[k].b.n ? 1 : 0);
+    n += (int)(dft_fwd_axes.size() + dft_adj_axes.size());
     n += (time_fwd.n_cta ? 1 : 0) + (time_adj.n_cta ? 1 : 0);
     n += (g_fwd.n_chunk ? 1 : 0) + 1;  // residual gather, threshold schedule
     if (wavelets) n += wav_fast ? 2 : 3;

@@ -24,7 +24,7 @@
 #include "kernels.cuh"
 #include "plan.hpp"
 #include "wavelet_fast.cuh"
-#include "line_dft.cuh"
+#include "plane_dft.cuh"
 #include "nn_api.hpp"
 #include "space_tc.cuh"
 

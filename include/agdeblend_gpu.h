@@ -54,7 +54,7 @@ void agd_gpu_problem_destroy(agd_gpu_problem *problem);
  * time-kernel candidates picked for the first time group (-1 without
  * one), [19] its number of candidates, [20] the wavelet-kernel candidate
  * picked (-1 without the prime-factor kernel), [21] their number, [22]
- * windows with one space axis on the line-DFT kernels (lengths without a
+ * windows with one space axis on the table-DFT kernels (lengths without a
  * shape-specialised kernel, up to 128). */
 int agd_gpu_problem_info(agd_gpu_problem const *problem, long int *info);
 

@@ -1,0 +1,103 @@
+"""The table-DFT space kernels (agdeblend_b200/csrc/plane_dft.cuh) of windows
+with two to four space axes: uneven windows (18 x 35 for a nominal 16 x 32),
+prime and even padded lengths, the shortest axes, the longest (128) and
+planes that fill the shared memory, three and four space axes (one or two
+single-axis passes beside the planes), windows on the shape-specialised
+kernels beside them.  Against the float64 oracle (operators: the gates of
+test_gpu_operators, 1e-5 relative L2 and the dot test in float, 1e-11 in
+double) and, for the update and its thresholds, the generic passes
+(AGD_GPU_GENERIC=1) over a solve."""
+import os
+
+import numpy as np
+import pytest
+
+import agdeblend_b200 as A
+from agdeblend_b200 import synthetic as S
+from conftest import rel_l2
+from test_gpu_operators import _check_operators
+
+pytestmark = pytest.mark.gpu
+
+
+def _survey(space, windows, nt=70, wt=32, seed=5):
+    """One patch with the given space shape and windows, one channel."""
+    rng = np.random.default_rng(seed)
+    n = int(np.prod(space))
+    st = np.cumsum(rng.integers(nt // 3, nt, n)).astype(np.int64)
+    tt = rng.choice([S.LIVE] * 8 + [S.BAD, S.MISSING], n).astype(np.int32)
+    tt[0] = S.LIVE
+    shape = [*space, nt]
+    data = rng.standard_normal(shape).astype(np.float32)
+    return S.Survey("plane", [0], [len(shape)], [[*windows, wt]], [[0] * len(space)], [shape],
+                    [st], [np.zeros(n, np.int32)], [tt], [data], [data.copy()], 12)
+
+
+# space shape, windows -> window lengths L (padded P) of the axes
+CASES = {
+    "uneven_18x35": ((37, 101), (16, 32)),      # L 18, 17 x 35, 34; P 23, 22 x 44, 43
+    "prime_P43x23": ((88, 28), (32, 16)),       # both windows uneven
+    "shortest": ((2, 3), (2, 3)),               # P 3 x 4
+    "short_and_long": ((3, 102), (3, 100)),     # P 4 x 128
+    "long_and_short": ((101, 5), (101, 5)),     # P 127 x 7
+    "largest_plane": ((90, 92), (90, 92)),      # P 113 x 115: one block per SM
+    "beside_fast_windows": ((16, 33), (16, 16)),  # 20 x 20 windows and uneven ones
+    "three_axes": ((9, 7, 11), (4, 7, 6)),
+    "three_axes_uneven_16": ((18, 17, 21), (16, 16, 16)),
+    "four_axes": ((5, 4, 6, 5), (4, 4, 6, 5)),
+}
+
+
+def _case(name):
+    space, windows = CASES[name]
+    return _survey(space, windows)
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_plane_operators_vs_oracle(name):
+    sv = _case(name)
+    prob = A.Problem.from_survey(sv)
+    assert prob.info[8] in (0, 2)
+    if prob.info[8] == 0:
+        k = prob.kernels()
+        assert k["space_fwd"] == k["space_adj"] and k["space_fwd"] in ("plane_dft", "line_dft")
+    prob.close()
+    _check_operators(sv, np.float32)
+
+
+@pytest.mark.parametrize("name", ["uneven_18x35", "shortest", "short_and_long",
+                                  "three_axes_uneven_16"])
+def test_plane_operators_double(name):
+    _check_operators(_case(name), np.float64, 1)
+
+
+def _solve(sv, generic):
+    old = os.environ.get("AGD_GPU_GENERIC")
+    os.environ["AGD_GPU_GENERIC"] = "1" if generic else "0"
+    try:
+        return A.deblend(sv.volumes, sv.window_shapes, sv.coords, sv.shottimes, sv.channels,
+                         sv.trace_types, 1.0, sv.n_its, 0, sv.data)
+    finally:
+        if old is None:
+            os.environ.pop("AGD_GPU_GENERIC", None)
+        else:
+            os.environ["AGD_GPU_GENERIC"] = old
+
+
+@pytest.mark.parametrize("name", ["uneven_18x35", "beside_fast_windows", "three_axes"])
+def test_plane_solve_matches_generic_passes(name):
+    sv = _case(name)
+    for o, r in zip(_solve(sv, False), _solve(sv, True)):
+        assert rel_l2(o, r) <= 1e-4
+
+
+def test_plane_batch_matches_separate_solves():
+    """Per-problem step, threshold and maximum in one launch."""
+    svs = [_survey((18, 35), (16, 32), seed=7), _survey((9, 11), (4, 6), seed=8),
+           _survey((37,), (16,), seed=9)]
+    kw = [dict(volumes=v.volumes, window_shapes=v.window_shapes, coords=v.coords,
+               shottimes=v.shottimes, channels=v.channels, trace_types=v.trace_types,
+               data=v.data) for v in svs]
+    for sv, out in zip(svs, A.deblend_batch(kw, 1.0, svs[0].n_its)):
+        for o, r in zip(out, _solve(sv, False)):
+            assert rel_l2(o, r) <= 1e-5
