@@ -109,6 +109,17 @@ __device__ __forceinline__ C mul_i(C a) {  // -i a (forward) or +i a (inverse)
   return INV ? cmake<C>(-a.y, a.x) : cmake<C>(a.y, -a.x);
 }
 
+// a + r b and a - r b for r = -i (forward) or +i (inverse): the components
+// cross over, so these stay scalar (a packed form would need them swapped)
+template <bool INV, typename C>
+__device__ __forceinline__ C add_rot(C a, C b) {
+  return INV ? cmake<C>(a.x - b.y, a.y + b.x) : cmake<C>(a.x + b.y, a.y - b.x);
+}
+template <bool INV, typename C>
+__device__ __forceinline__ C sub_rot(C a, C b) {
+  return INV ? cmake<C>(a.x + b.y, a.y - b.x) : cmake<C>(a.x - b.y, a.y + b.x);
+}
+
 __host__ __device__ constexpr int small_split(int n) {
   // largest explicit radix that divides n with a nontrivial cofactor
   return (n % 8 == 0 && n > 8) ? 8
@@ -171,18 +182,11 @@ __device__ __forceinline__ void dft_odd(Cx<R> (&v)[N]) {
 #pragma unroll
     for (int j = 1; j <= H; ++j) {
       const C w = ctw<R>(off + (j * k) % N);  // (cos, -sin) of 2 pi j k / N
-      a.x += sum[j - 1].x * w.x;
-      a.y += sum[j - 1].y * w.x;
-      b.x -= dif[j - 1].x * w.y;
-      b.y -= dif[j - 1].y * w.y;
+      a = cfma(a, w.x, sum[j - 1]);
+      b = cfma(b, -w.y, dif[j - 1]);
     }
-    if (INV) {
-      v[k] = cmake<C>(a.x - b.y, a.y + b.x);
-      v[N - k] = cmake<C>(a.x + b.y, a.y - b.x);
-    } else {
-      v[k] = cmake<C>(a.x + b.y, a.y - b.x);
-      v[N - k] = cmake<C>(a.x - b.y, a.y + b.x);
-    }
+    v[k] = add_rot<INV>(a, b);
+    v[N - k] = sub_rot<INV>(a, b);
   }
   v[0] = tot;
 }
@@ -255,20 +259,20 @@ __device__ __forceinline__ void dft(Cx<R> (&v)[N]) {
   } else if constexpr (N == 3) {
     const R c = (R)0.86602540378443864676;
     const C t1 = cadd(v[1], v[2]);
-    const C t2 = cmake<C>(v[0].x - (R)0.5 * t1.x, v[0].y - (R)0.5 * t1.y);
-    const C t3 = mul_i<INV>(cscale(csub(v[1], v[2]), c));
+    const C t2 = cfma(v[0], (R)-0.5, t1);
+    const C t3 = cscale(csub(v[1], v[2]), c);
     v[0] = cadd(v[0], t1);
-    v[1] = cadd(t2, t3);
-    v[2] = csub(t2, t3);
+    v[1] = add_rot<INV>(t2, t3);
+    v[2] = sub_rot<INV>(t2, t3);
   } else if constexpr (N == 4) {
     const C s02 = cadd(v[0], v[2]);
     const C d02 = csub(v[0], v[2]);
     const C s13 = cadd(v[1], v[3]);
-    const C r13 = mul_i<INV>(csub(v[1], v[3]));
+    const C d13 = csub(v[1], v[3]);
     v[0] = cadd(s02, s13);
-    v[1] = cadd(d02, r13);
+    v[1] = add_rot<INV>(d02, d13);
     v[2] = csub(s02, s13);
-    v[3] = csub(d02, r13);
+    v[3] = sub_rot<INV>(d02, d13);
   } else if constexpr (N == 5) {
     const R c1 = (R)0.30901699437494742410;
     const R c2 = (R)-0.80901699437494742410;
@@ -278,15 +282,15 @@ __device__ __forceinline__ void dft(Cx<R> (&v)[N]) {
     const C t2 = cadd(v[2], v[3]);
     const C t3 = csub(v[1], v[4]);
     const C t4 = csub(v[2], v[3]);
-    const C a1 = cmake<C>(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
-    const C a2 = cmake<C>(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
-    const C b1 = mul_i<INV>(cmake<C>(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y));
-    const C b2 = mul_i<INV>(cmake<C>(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y));
+    const C a1 = cfma(cfma(v[0], c1, t1), c2, t2);
+    const C a2 = cfma(cfma(v[0], c2, t1), c1, t2);
+    const C b1 = cfma(cscale(t3, s1), s2, t4);
+    const C b2 = cfma(cscale(t3, s2), -s1, t4);
     v[0] = cadd(v[0], cadd(t1, t2));
-    v[1] = cadd(a1, b1);
-    v[4] = csub(a1, b1);
-    v[2] = cadd(a2, b2);
-    v[3] = csub(a2, b2);
+    v[1] = add_rot<INV>(a1, b1);
+    v[4] = sub_rot<INV>(a1, b1);
+    v[2] = add_rot<INV>(a2, b2);
+    v[3] = sub_rot<INV>(a2, b2);
   } else if constexpr (N == 8) {
     // even/odd split into two 4-point DFTs, W_8 = (1 -/+ i) / sqrt(2)
     C e[4] = {v[0], v[2], v[4], v[6]};
@@ -294,17 +298,14 @@ __device__ __forceinline__ void dft(Cx<R> (&v)[N]) {
     dft<R, 4, INV>(e);
     dft<R, 4, INV>(o);
     const R h = (R)0.70710678118654752440;
-    const C o1 = INV ? cmake<C>(h * (o[1].x - o[1].y), h * (o[1].x + o[1].y))
-                     : cmake<C>(h * (o[1].x + o[1].y), h * (o[1].y - o[1].x));
-    const C o2 = mul_i<INV>(o[2]);
-    const C o3 = INV ? cmake<C>(-h * (o[3].x + o[3].y), h * (o[3].x - o[3].y))
-                     : cmake<C>(h * (o[3].y - o[3].x), -h * (o[3].x + o[3].y));
+    const C o1 = cscale(add_rot<INV>(o[1], o[1]), h);  // W_8 o_1 = h (1 +/- i) o_1
+    const C o3 = cscale(sub_rot<INV>(o[3], o[3]), -h);
     v[0] = cadd(e[0], o[0]);
     v[4] = csub(e[0], o[0]);
     v[1] = cadd(e[1], o1);
     v[5] = csub(e[1], o1);
-    v[2] = cadd(e[2], o2);
-    v[6] = csub(e[2], o2);
+    v[2] = add_rot<INV>(e[2], o[2]);
+    v[6] = sub_rot<INV>(e[2], o[2]);
     v[3] = cadd(e[3], o3);
     v[7] = csub(e[3], o3);
   } else if constexpr (coprime_split(N) != 0) {

@@ -54,6 +54,40 @@ template <typename C>
 __device__ __forceinline__ C csub(C a, C b) {
   return cmake<C>(a.x - b.x, a.y - b.y);
 }
+// Single precision: one packed instruction on the (x, y) pair (the rate of
+// the FP32 pipe is the same, the issue slots are half; rounding per element
+// as the scalar operations).
+__device__ __forceinline__ unsigned long long pack2(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(r);
+}
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(r);
+}
+// a + s b for a real s
+__device__ __forceinline__ float2 cfma(float2 a, float s, float2 b) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r)
+      : "l"(pack2(make_float2(s, s))), "l"(pack2(b)), "l"(pack2(a)));
+  return unpack2(r);
+}
+__device__ __forceinline__ double2 cfma(double2 a, double s, double2 b) {
+  return make_double2(a.x + s * b.x, a.y + s * b.y);
+}
 template <typename C>
 __device__ __forceinline__ C cmul(C a, C b) {
   return cmake<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -61,6 +95,11 @@ __device__ __forceinline__ C cmul(C a, C b) {
 template <typename C>
 __device__ __forceinline__ C cscale(C a, decltype(C{}.x) s) {
   return cmake<C>(a.x * s, a.y * s);
+}
+__device__ __forceinline__ float2 cscale(float2 a, float s) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(make_float2(s, s))));
+  return unpack2(r);
 }
 // multiply by -i (forward) or +i (inverse)
 template <typename C>
