@@ -178,9 +178,9 @@ int agd_gpu_problem_info(agd_gpu_problem const *pb, long int *info) {
   info[14] = e.kernels_per_iteration();
   info[15] = (long)e.classes.size();
   info[16] = n_fast;
-  info[17] = e.tgroups.empty() ? -1 : e.tgroups[0]->fwd_pick;
-  info[18] = e.tgroups.empty() ? -1 : e.tgroups[0]->adj_pick;
-  info[19] = e.tgroups.empty() ? 0 : (long)e.tgroups[0]->fwd_vars.size();
+  info[17] = e.tgroups.empty() ? -1 : 0;
+  info[18] = e.tgroups.empty() ? -1 : 0;
+  info[19] = e.tgroups.empty() ? 0 : 1;
   info[20] = e.wav_fast ? e.wav_pick : -1;
   info[21] = e.wav_candidates;
   long n_line = 0;
@@ -201,7 +201,7 @@ int agd_gpu_problem_kernels(agd_gpu_problem const *pb, char *buf, int len) {
       buf, (size_t)len, "space_fwd=%s space_adj=%s time_fwd=%s time_adj=%s wavelet=%s",
       !sc ? other : (e.classes[0]->tc ? "space_fwd_tc" : e.classes[0]->fv().name),
       !sc ? other : (e.classes[0]->tc ? "space_adj_tc" : e.classes[0]->av().name),
-      tg ? e.tgroups[0]->fv().name : "time_c2r_ola", tg ? e.tgroups[0]->av().name : "time_r2c",
+      tg ? "time_fwd_pair" : "time_c2r_ola", tg ? "time_adj_pair" : "time_r2c",
       !e.wavelets ? "none" : (e.wav_fast ? "wavelet_fast" : "wavelet_apply"));
   return n < 0 || n >= len ? 1 : 0;
 }

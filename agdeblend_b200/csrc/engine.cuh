@@ -26,6 +26,7 @@ class Engine {
     DevArray<int> cta_trace0;
     int n_cta = 0;
     int nb = 0;
+    int splits = 1;  // shares of the time windows (trace-pair kernels)
     size_t smem = 0;
   };
   struct GatherLaunch {
@@ -132,29 +133,14 @@ class Engine {
     const FwdVariant &fv() const { return fwd_vars[fwd_pick]; }
     const AdjVariant &av() const { return adj_vars[adj_pick]; }
   };
-  // windows of one padded time length on the fast time kernels (whatever
-  // kernels serve their space axes), with candidate instantiations (traces
-  // per block, padded line stride, blocks per SM) picked by timing
-  struct TimeFwdVariant {
-    TimeFwdFn fn;
-    int nb;
-    size_t smem;
-    const char *name;  // kernel family (as profilers list it)
-  };
-  struct TimeAdjVariant {
-    TimeAdjFn fn;
-    int nb;
-    size_t smem;
-    const char *name;  // kernel family (as profilers list it)
-  };
+  // windows of one padded time length on the trace-pair time kernels
+  // (time_pair.cuh), whatever kernels serve their space axes
   struct TimeGroup {
     std::vector<int> win;
-    std::vector<TimeFwdVariant> fwd_vars;
-    std::vector<TimeAdjVariant> adj_vars;
-    int fwd_pick = 0, adj_pick = 0;
+    TimeFwdFn fwd = nullptr;
+    TimeAdjFn adj = nullptr;
+    size_t fwd_smem = 0, adj_smem = 0;
     TimeLaunch tf, ta;
-    const TimeFwdVariant &fv() const { return fwd_vars[fwd_pick]; }
-    const TimeAdjVariant &av() const { return adj_vars[adj_pick]; }
   };
   std::vector<std::unique_ptr<FastClass>> classes;
   std::vector<std::unique_ptr<TimeGroup>> tgroups;
@@ -826,64 +812,30 @@ class Engine {
     return !c.fwd_vars.empty() && !c.adj_vars.empty();
   }
 
-  // time-axis kernel candidates for Pt = 2 M1 M2: NB traces per block, line
-  // stride LS (M + 1, or padded to 10 mod 16 complex so that the four-step
-  // passes hit distinct banks), MB blocks per SM
-  template <int M1, int M2, int NB, int LS, int MB>
-  static void add_time(TimeGroup &g) {
-    constexpr int M = M1 * M2;
-    constexpr int H = 4 * M / 5;
-    g.fwd_vars.push_back(TimeFwdVariant{time_fwd_fast<R, M1, M2, NB, LS, MB>, NB,
-                                        2 * (size_t)NB * LS * sizeof(C) +
-                                            (size_t)NB * H * sizeof(R), "time_fwd_fast"});
-    g.adj_vars.push_back(TimeAdjVariant{time_adj_fast<R, M1, M2, NB, LS, MB>, NB,
-                                        (size_t)NB * LS * sizeof(C) +
-                                            2 * (size_t)NB * 2 * H * sizeof(R), "time_adj_fast"});
-  }
+  // blocks per SM that the trace-pair time kernels are compiled for
+  static constexpr int kPairBlocks = sizeof(R) == sizeof(float) ? 4 : 2;
 
-  // fused candidates (fast.cuh time_fwd_fused / time_adj_fused), 256 / M1
-  // traces per block
-  template <int M1, int M2, int LSB, int LSW, int MB>
-  static void add_time_fused(TimeGroup &g) {
-    constexpr int M = M1 * M2;
-    constexpr int H = 4 * M / 5;
-    constexpr int NB = kThreads / M1;
-    g.fwd_vars.push_back(TimeFwdVariant{time_fwd_fused<R, M1, M2, LSB, LSW, MB>, NB,
-                                        ((size_t)2 * NB * LSB + (size_t)NB * LSW) * sizeof(C), "time_fwd_fused"});
-    constexpr int LT = 2 * H;
-    constexpr int LTP = LT + ((20 - LT % 32) + 32) % 32;  // as time_adj_fused
-    g.adj_vars.push_back(TimeAdjVariant{time_adj_fused<R, M1, M2, LSW, MB>, NB,
-                                        (size_t)NB * LSW * sizeof(C) +
-                                            2 * (size_t)NB * LTP * sizeof(R), "time_adj_fused"});
+  template <int NA>
+  static void set_time_kernels(TimeGroup &g) {
+    using S = TimePair<R, NA>;
+    g.fwd = time_fwd_pair<R, NA, kPairBlocks>;
+    g.adj = time_adj_pair<R, NA, kPairBlocks>;
+    g.fwd_smem = S::kFwdSmem;
+    g.adj_smem = S::kAdjSmem;
   }
 
   static bool time_case(const WindowPlan &W, TimeGroup &g) {
-    g.fwd_vars.clear();
-    g.adj_vars.clear();
-    if (W.Pt == 320) {
-      add_time<16, 10, 32, 161, 1>(g);
-      if constexpr (sizeof(R) == sizeof(float)) {
-        add_time<16, 10, 32, 170, 2>(g);
-        add_time<16, 10, 16, 170, 4>(g);
-        add_time_fused<16, 10, 170, 186, 3>(g);
-        add_time_fused<16, 10, 170, 186, 2>(g);
-      }
-    } else if (W.Pt == 160) {
-      add_time<8, 10, 32, 81, 1>(g);
-      if constexpr (sizeof(R) == sizeof(float)) {
-        add_time<8, 10, 32, 90, 2>(g);
-        add_time<8, 10, 16, 90, 4>(g);
-        add_time_fused<8, 10, 90, 90, 3>(g);
-        add_time_fused<8, 10, 90, 90, 2>(g);
-      }
-    } else {
+    if (W.Pt == 320)
+      set_time_kernels<16>(g);
+    else if (W.Pt == 160)
+      set_time_kernels<8>(g);
+    else
       return false;
-    }
     return true;
   }
 
-  // the fast space kernels assume L = 4P/5 on every space axis, the fast
-  // time kernels Lt = 2h = 4Pt/5
+  // the fast space kernels assume L = 4P/5 on every space axis, the
+  // trace-pair time kernels Lt = 2h = 4Pt/5
   static bool space_eligible(const WindowPlan &W) {
     for (int d = 0; d < W.D; ++d)
       if (W.L[d] * 5 != W.P[d] * 4) return false;
@@ -1337,8 +1289,7 @@ class Engine {
     const int limit = optin_smem();
     int dyn = smem_max;
     for (const auto &gp : tgroups) {
-      for (const TimeFwdVariant &v : gp->fwd_vars) dyn = std::min(dyn, opt_in(v.fn, limit));
-      for (const TimeAdjVariant &v : gp->adj_vars) dyn = std::min(dyn, opt_in(v.fn, limit));
+      dyn = std::min({dyn, opt_in(gp->fwd, limit), opt_in(gp->adj, limit)});
     }
     for (const auto &cp : classes) {
       for (const FwdVariant &v : cp->fwd_vars) dyn = std::min(dyn, opt_in(v.fn, limit));
@@ -1531,117 +1482,44 @@ class Engine {
     if (h) throw DeviceError("a tensor-core kernel gave up waiting for its MMAs");
   }
 
+  // Blocks of 2 kPairs traces over the group's windows, and the number of
+  // shares that the time windows are split into: the least number of windows
+  // that the longest-running SM walks one after another (a forward share
+  // repeats the window before it, an adjoint share loads half of one more).
+  // Surveys whose blocks fill the device (98 windows of 512 traces: 3136
+  // blocks) are not split; a 128-trace gather (14 blocks of 5 windows) is,
+  // into one window per block: 14 blocks of five windows took 17 us forward
+  // and 20 us adjoint, 70 blocks take 11 and 10 us.
   void build_time_group(TimeGroup &g) {
-    autotune_time(g);
-    make_fixed_time_launch(g.tf, g.fv().smem, g.win, g.fv().nb);
-    make_fixed_time_launch(g.ta, g.av().smem, g.win, g.av().nb);
-  }
-
-  // As autotune_space, for the candidates of a time group: forward
-  // S0/S1 -> Y, adjoint record (or Y after the wavelet stage) -> S0/S1.
-  // AGD_GPU_TIME_VARIANT="f,a" forces the candidates (tests).
-  void autotune_time(TimeGroup &g) {
-    g.fwd_pick = g.adj_pick = 0;
-    const char *env = std::getenv("AGD_GPU_TIME_VARIANT");
-    if (env != nullptr && env[0] != '\0') {
-      int f = 0, a = 0;
-      if (std::sscanf(env, "%d,%d", &f, &a) == 2) {
-        g.fwd_pick = std::max(0, std::min(f, (int)g.fwd_vars.size() - 1));
-        g.adj_pick = std::max(0, std::min(a, (int)g.adj_vars.size() - 1));
-        return;
-      }
-    }
-    if (g.fwd_vars.size() == 1 && g.adj_vars.size() == 1) return;
-    long traces = 0;
-    for (int w : g.win) traces += plan.windows[w].n_traces;
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
-    char key[96];
-    std::snprintf(key, sizeof key, "time:%d:%d:%d:%d:%d", dev, (int)sizeof(R),
-                  plan.windows[g.win[0]].Pt, wavelets ? 1 : 0,
-                  (int)std::log2((double)std::max(1L, traces)));
-    static std::mutex mu;
-    static std::map<std::string, std::pair<int, int>> cache;
-    {
-      std::lock_guard<std::mutex> lk(mu);
-      auto it = cache.find(key);
-      if (it != cache.end()) {
-        g.fwd_pick = it->second.first;
-        g.adj_pick = it->second.second;
-        return;
-      }
-    }
-    if (Y.get() != nullptr) CK(cudaMemsetAsync(Y.get(), 0, Y.bytes(), stream));
-    if (rec_d.get() != nullptr) CK(cudaMemsetAsync(rec_d.get(), 0, rec_d.bytes(), stream));
-    cudaEvent_t e0, e1;
-    CK(cudaEventCreate(&e0));
-    CK(cudaEventCreate(&e1));
-    auto timed = [&](auto launch) {
-      launch();
-      CK(cudaEventRecord(e0, stream));
-      launch();
-      launch();
-      CK(cudaEventRecord(e1, stream));
-      CK(cudaEventSynchronize(e1));
-      float ms = 0;
-      CK(cudaEventElapsedTime(&ms, e0, e1));
-      return ms;
-    };
-    const size_t nf = g.fwd_vars.size(), na = g.adj_vars.size();
-    std::vector<TimeLaunch> lf(nf), la(na);
-    std::vector<float> tf(nf, 1e30f), ta(na, 1e30f);
-    for (size_t v = 0; v < nf; ++v)
-      if (g.fwd_vars[v].smem <= (size_t)smem_max)
-        make_fixed_time_launch(lf[v], g.fwd_vars[v].smem, g.win, g.fwd_vars[v].nb);
-    for (size_t v = 0; v < na; ++v)
-      if (g.adj_vars[v].smem <= (size_t)smem_max)
-        make_fixed_time_launch(la[v], g.adj_vars[v].smem, g.win, g.adj_vars[v].nb);
-    const int from_record = wavelets ? 0 : 1;
-    for (int round = 0; round < 3; ++round) {
-      for (size_t v = 0; v < nf; ++v) {
-        const TimeLaunch &L = lf[v];
-        if (L.n_cta == 0) continue;
-        const TimeFwdFn fn = g.fwd_vars[v].fn;
-        tf[v] = std::min(tf[v], timed([&] {
-          fn<<<L.n_cta, kThreads, L.smem, stream>>>(time_jobs.get(), L.cta_job.get(),
-                                                    L.cta_trace0.get());
-          CK(cudaGetLastError());
-        }));
-      }
-      for (size_t v = 0; v < na; ++v) {
-        const TimeLaunch &L = la[v];
-        if (L.n_cta == 0) continue;
-        const TimeAdjFn fn = g.adj_vars[v].fn;
-        ta[v] = std::min(ta[v], timed([&] {
-          fn<<<L.n_cta, kThreads, L.smem, stream>>>(time_jobs.get(), L.cta_job.get(),
-                                                    L.cta_trace0.get(), rec_d.get(),
-                                                    from_record);
-          CK(cudaGetLastError());
-        }));
-      }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    g.fwd_pick = (int)(std::min_element(tf.begin(), tf.end()) - tf.begin());
-    g.adj_pick = (int)(std::min_element(ta.begin(), ta.end()) - ta.begin());
-    std::lock_guard<std::mutex> lk(mu);
-    cache[key] = {g.fwd_pick, g.adj_pick};
-  }
-
-  void make_fixed_time_launch(TimeLaunch &L, size_t smem, const std::vector<int> &wins,
-                              int nb) {
-    if (smem > (size_t)smem_max) throw DeviceError("time window too long for shared memory");
+    if (std::max(g.fwd_smem, g.adj_smem) > (size_t)smem_max)
+      throw DeviceError("time window too long for shared memory");
     std::vector<int> cj, ct;
-    for (int w : wins)
-      for (int t = 0; t < plan.windows[w].n_traces; t += nb) {
+    int T = 1;
+    for (int w : g.win) {
+      T = std::max(T, plan.windows[w].T);
+      for (int t = 0; t < plan.windows[w].n_traces; t += 2 * kPairs) {
         cj.push_back(w);
         ct.push_back(t);
       }
-    L.cta_job.upload(cj, stream);
-    L.cta_trace0.upload(ct, stream);
-    L.n_cta = (int)cj.size();
-    L.nb = nb;
-    L.smem = smem;
+    }
+    for (bool fwd : {true, false}) {
+      TimeLaunch &L = fwd ? g.tf : g.ta;
+      L.cta_job.upload(cj, stream);
+      L.cta_trace0.upload(ct, stream);
+      L.n_cta = (int)cj.size();
+      L.nb = 2 * kPairs;
+      L.smem = fwd ? g.fwd_smem : g.adj_smem;
+      const long resident = (long)kPairBlocks * n_sm;
+      double best = 1e300;
+      for (int s = 1; s <= std::min(T, 64); ++s) {
+        const double walk = (T + s - 1) / s + (s > 1 ? (fwd ? 1.0 : 0.5) : 0.0);
+        const double cost = (double)((L.n_cta * (long)s + resident - 1) / resident) * walk;
+        if (cost < best - 1e-9) {
+          best = cost;
+          L.splits = s;
+        }
+      }
+    }
   }
 
   void make_gather(GatherLaunch &G, const std::vector<Contrib> &list, long record_size) {
@@ -2028,8 +1906,8 @@ class Engine {
     for (const auto &gp : tgroups) {
       const TimeGroup &g = *gp;
       if (!g.tf.n_cta) continue;
-      g.fv().fn<<<g.tf.n_cta, kThreads, g.tf.smem, stream>>>(time_jobs.get(), g.tf.cta_job.get(),
-                                                             g.tf.cta_trace0.get());
+      g.fwd<<<dim3(g.tf.n_cta, g.tf.splits), kPairThreads, g.tf.smem, stream>>>(
+          time_jobs.get(), g.tf.cta_job.get(), g.tf.cta_trace0.get());
       CK(cudaGetLastError());
     }
     if (time_fwd.n_cta) {
@@ -2046,7 +1924,7 @@ class Engine {
     for (const auto &gp : tgroups) {
       const TimeGroup &g = *gp;
       if (!g.ta.n_cta) continue;
-      g.av().fn<<<g.ta.n_cta, kThreads, g.ta.smem, stream>>>(
+      g.adj<<<dim3(g.ta.n_cta, g.ta.splits), kPairThreads, g.ta.smem, stream>>>(
           time_jobs.get(), g.ta.cta_job.get(), g.ta.cta_trace0.get(), record, from_record);
       CK(cudaGetLastError());
     }

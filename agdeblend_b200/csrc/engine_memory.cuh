@@ -25,6 +25,7 @@
 #include "plan.hpp"
 #include "wavelet_fast.cuh"
 #include "plane_dft.cuh"
+#include "time_pair.cuh"
 #include "nn_api.hpp"
 #include "space_tc.cuh"
 

@@ -1,8 +1,8 @@
 // Shape-specialised kernels of the deblending operator for sm_100a.
 //
 // Every FFT here runs in registers with a compile-time size: a thread owns a
-// whole line (space axes) or one factor of a four-step transform (time axis),
-// so the radix schedule, the index arithmetic and the twiddle offsets are
+// whole line (or, in time_pair.cuh, one factor of a four-step transform), so
+// the radix schedule, the index arithmetic and the twiddle offsets are
 // constants.  Lengths with coprime factors (20 = 4 * 5, 40 = 8 * 5, 10 = 2 * 5)
 // use the prime-factor split, which needs no twiddles; the other twiddles
 // live in __constant__ memory (filled once per device from double-precision
@@ -15,12 +15,7 @@
 //                   axis, then x <- soft_threshold(x - step * g, lambda);
 //   space_adj_pipe  the adjoint with the next batch's input copied into a
 //                   dense staging buffer behind the passes, and the update
-//                   keeping several model loads in flight;
-//   time_fwd_fast   per block of traces, every time window: Hermitian
-//                   combine, half-length inverse FFT (four-step in shared
-//                   memory), taper, overlap-add with a one-hop carry;
-//   time_adj_fast   per block of traces, every time window: gather from the
-//                   record, taper, half-length forward FFT, split, double.
+//                   keeping several model loads in flight.
 //
 // Kernels for other sizes are the generic ones in kernels.cuh.
 #pragma once
@@ -1116,565 +1111,6 @@ __global__ void __launch_bounds__(NT, MINB)
     __shared__ R red[32];
     const R m = block_max<R>(local_max, red);
     if (threadIdx.x == 0) atomic_max_nonneg(max_out, m);
-  }
-}
-
-// ------------------------------------------------------------ time axis
-
-// Twiddles W_N^k, k < N, copied to shared memory for lookups whose index
-// differs between threads (constant memory serialises such accesses).
-template <typename R, int N>
-__device__ __forceinline__ void load_twiddles(Cx<R> *tw) {
-  for (int k = threadIdx.x; k < N; k += blockDim.x) tw[k] = ctw<R>(tw_offset(N) + k);
-}
-
-template <bool INV, typename C>
-__device__ __forceinline__ C tw_at(const C *tw, int k) {
-  C w = tw[k];
-  if (INV) w.y = -w.y;
-  return w;
-}
-
-// Four-step FFT of length M = M1 * M2 on nl lines of shared memory (line
-// stride LS), twiddles W_M from shared memory.  Output X[k1 + M1 k2] is left
-// at position M2 k1 + k2.
-template <typename R, int M1, int M2, bool INV>
-__device__ __forceinline__ void lines_fourstep(Cx<R> *buf, int nl, int LS, const Cx<R> *twM) {
-  using C = Cx<R>;
-  constexpr int M = M1 * M2;
-  for (int w = threadIdx.x; w < nl * M2; w += blockDim.x) {
-    const int line = w / M2;
-    const int n2 = w - line * M2;
-    C *b = buf + line * LS;
-    C v[M1];
-#pragma unroll
-    for (int n1 = 0; n1 < M1; ++n1) v[n1] = b[M2 * n1 + n2];
-    dft<R, M1, INV>(v);
-#pragma unroll
-    for (int k1 = 0; k1 < M1; ++k1)
-      b[M2 * k1 + n2] = (k1 == 0) ? v[0] : cmul(v[k1], tw_at<INV>(twM, (n2 * k1) % M));
-  }
-  __syncthreads();
-  for (int w = threadIdx.x; w < nl * M1; w += blockDim.x) {
-    const int line = w / M1;
-    const int k1 = w - line * M1;
-    C *b = buf + line * LS + M2 * k1;
-    C v[M2];
-#pragma unroll
-    for (int n2 = 0; n2 < M2; ++n2) v[n2] = b[n2];
-    dft<R, M2, INV>(v);
-#pragma unroll
-    for (int k2 = 0; k2 < M2; ++k2) b[k2] = v[k2];
-  }
-  __syncthreads();
-}
-
-template <int M1, int M2>
-__device__ __forceinline__ int fourstep_pos(int k) {
-  return M2 * (k % M1) + k / M1;
-}
-
-// Forward time axis for Pt = 2 M (M = M1 M2) and Lt = 2 h with h = 4 M / 5
-// (the window length whose padded length is Pt): per trace and time window,
-// c2r of the F = M + 1 bins through a length-M complex FFT, then taper and
-// overlap-add; segment [t h, (t+1) h) of a trace is final once window t is
-// added, so only a one-hop carry stays in shared memory.  Blocks own NB
-// traces; the bins of window t + 1 are copied in (cp.async) while window t is
-// processed.  Lines of the F = M + 1 bins are LS >= F apart in shared memory
-// (a padded stride spreads the four-step accesses over the banks); MINB
-// blocks share an SM.
-template <typename R, int M1, int M2, int NB, int LS, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB)
-    time_fwd_fast(const TimeJob<R> *__restrict__ jobs, const int *__restrict__ cta_job,
-                  const int *__restrict__ cta_trace0) {
-  using C = Cx<R>;
-  constexpr int M = M1 * M2;
-  constexpr int F = M + 1;  // bins per line
-  static_assert(LS >= F, "line stride");
-  constexpr int H = 4 * M / 5;
-  constexpr int HALF = M / 2 + 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ C twM[M];
-  __shared__ C tw2M[2 * M];
-  __shared__ R taper[2 * H];
-  __shared__ R scale[NB];
-  load_twiddles<R, M>(twM);
-  load_twiddles<R, 2 * M>(tw2M);
-  const TimeJob<R> job = jobs[cta_job[blockIdx.x]];
-  const int t0 = cta_trace0[blockIdx.x];
-  const int nb = min(NB, job.n_traces - t0);
-  const long ntr = job.n_traces;
-  for (int j = threadIdx.x; j < 2 * H; j += kThreads) taper[j] = job.time_taper[j];
-  for (int i = threadIdx.x; i < NB; i += kThreads) scale[i] = i < nb ? job.space_scale[t0 + i] : (R)0;
-  C *stage[2] = {reinterpret_cast<C *>(smem_raw), reinterpret_cast<C *>(smem_raw) + NB * LS};
-  R *carry = reinterpret_cast<R *>(stage[1] + NB * LS);  // [NB][H]
-  auto issue = [&](int t, C *buf) {
-    const C *zt = job.z + (long)t * F * ntr + t0;
-    for (int idx = threadIdx.x; idx < NB * F; idx += kThreads) {
-      const int f = idx / NB;
-      const int i = idx - f * NB;
-      if (i < nb) cp_async<sizeof(C)>(buf + i * LS + f, zt + f * ntr + i);
-    }
-  };
-  for (int i = threadIdx.x; i < NB * H; i += kThreads) carry[i] = (R)0;
-  issue(0, stage[0]);
-  cp_async_commit();
-  for (int t = 0; t < job.T; ++t) {
-    if (t + 1 < job.T) issue(t + 1, stage[(t + 1) & 1]);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    C *buf = stage[t & 1];
-    // Hermitian combine into M complex values (pairs k, M - k per thread):
-    // Z_k = (X_k + conj X_{M-k}) + i e^{+2 pi i k / Pt} (X_k - conj X_{M-k})
-    for (int w = threadIdx.x; w < NB * HALF; w += kThreads) {
-      const int i = w / HALF;
-      const int k = w - i * HALF;
-      C *b = buf + i * LS;
-      const int kk = M - k;
-      C xa = b[k];
-      C xb = b[kk];
-      if (k == 0) {
-        xa.y = (R)0;
-        xb.y = (R)0;
-      }
-      auto comb = [&](C a, C bc_src, int kidx) {
-        const C bc = cmake<C>(bc_src.x, -bc_src.y);
-        const C e = cadd(a, bc);
-        const C d = csub(a, bc);
-        const C o = cmul(d, tw_at<true>(tw2M, kidx));
-        return cmake<C>(e.x - o.y, e.y + o.x);
-      };
-      const C za = comb(xa, xb, k);
-      if (k != 0 && k != kk) b[kk] = comb(xb, xa, kk);
-      b[k] = za;  // k == 0 pairs with the Nyquist bin, which is then unused
-    }
-    __syncthreads();
-    lines_fourstep<R, M1, M2, true>(buf, NB, LS, twM);
-    // taper, overlap-add, write the completed segment of each trace; one
-    // thread owns samples j and j + H, so the carry is read then rewritten
-    // by the same thread
-    for (int idx = threadIdx.x; idx < NB * H; idx += kThreads) {
-      const int i = idx / H;
-      const int j = idx - i * H;
-      if (i < nb) {
-        const R sc = scale[i];
-        const C z_lo = buf[i * LS + fourstep_pos<M1, M2>(j >> 1)];
-        const C z_hi = buf[i * LS + fourstep_pos<M1, M2>((j + H) >> 1)];
-        const R u_lo = (j & 1) ? z_lo.y : z_lo.x;
-        const R u_hi = ((j + H) & 1) ? z_hi.y : z_hi.x;
-        job.y[(long)(t0 + i) * job.C + t * H + j] = carry[idx] + (u_lo * sc) * taper[j];
-        carry[idx] = (u_hi * sc) * taper[j + H];
-      }
-    }
-    __syncthreads();
-  }
-  // last half window and the zero tail up to C
-  for (int idx = threadIdx.x; idx < NB * H; idx += kThreads) {
-    const int i = idx / H;
-    if (i < nb) job.y[(long)(t0 + i) * job.C + job.T * H + (idx - i * H)] = carry[idx];
-  }
-  const int tail = job.C - (job.T + 1) * H;
-  for (int idx = threadIdx.x; idx < nb * tail; idx += kThreads) {
-    const int i = idx / tail;
-    const int j = idx - i * tail;
-    job.y[(long)(t0 + i) * job.C + (job.T + 1) * H + j] = (R)0;
-  }
-}
-
-// Adjoint time axis for Pt = 2 M and Lt = 2 h, h = 4 M / 5: per trace and
-// window, gather Lt samples (record through the blend coordinates, or the
-// trace buffer), taper, pack pairs into M complex values, forward FFT, split
-// into the M + 1 bins and double bins 1..M-1.  The raw samples of window
-// t + 1 are copied in (cp.async, zero-filled outside the blended span) while
-// window t is transformed.  Line stride LS >= M + 1 and MINB as in
-// time_fwd_fast.
-template <typename R, int M1, int M2, int NB, int LS, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB)
-    time_adj_fast(const TimeJob<R> *__restrict__ jobs, const int *__restrict__ cta_job,
-                  const int *__restrict__ cta_trace0, const R *__restrict__ record,
-                  int from_record) {
-  using C = Cx<R>;
-  constexpr int M = M1 * M2;
-  constexpr int F = M + 1;  // bins per line
-  static_assert(LS >= F, "line stride");
-  constexpr int H = 4 * M / 5;
-  constexpr int LT = 2 * H;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ C twM[M];
-  __shared__ C tw2M[2 * M];
-  __shared__ long span_base[NB];  // source index of trace sample 0
-  __shared__ int span_lo[NB], span_hi[NB];  // readable trace samples [lo, hi)
-  __shared__ R scale[NB];
-  __shared__ R taper[LT];
-  load_twiddles<R, M>(twM);
-  load_twiddles<R, 2 * M>(tw2M);
-  const TimeJob<R> job = jobs[cta_job[blockIdx.x]];
-  const int t0 = cta_trace0[blockIdx.x];
-  const int nb = min(NB, job.n_traces - t0);
-  const long ntr = job.n_traces;
-  for (int j = threadIdx.x; j < LT; j += kThreads) taper[j] = job.time_taper[j];
-  for (int i = threadIdx.x; i < NB; i += kThreads) {
-    const int tr = t0 + i;
-    span_lo[i] = 0;
-    span_hi[i] = 0;
-    span_base[i] = 0;
-    scale[i] = (R)0;
-    if (i >= nb) continue;
-    scale[i] = job.space_scale[tr];
-    if (from_record) {
-      const long rec = job.blend_rec[tr];
-      const int ts = job.blend_ts[tr];
-      span_base[i] = rec - ts;
-      span_lo[i] = rec >= 0 ? ts : 0;
-      span_hi[i] = rec >= 0 ? ts + job.blend_n[tr] : 0;
-    } else {
-      span_base[i] = (long)tr * job.C;
-      span_hi[i] = job.C;
-    }
-  }
-  __syncthreads();
-  const R *src_base = from_record ? record : job.y;
-  C *line = reinterpret_cast<C *>(smem_raw);
-  R *raw[2] = {reinterpret_cast<R *>(line + NB * LS), reinterpret_cast<R *>(line + NB * LS) + NB * LT};
-  auto issue = [&](int t, R *rb) {
-    // four consecutive samples per thread and step
-    for (int g = threadIdx.x; g < NB * (LT / 4); g += kThreads) {
-      const int i = g / (LT / 4);
-      const int j0 = 4 * (g - i * (LT / 4));
-      const int s0 = t * H + j0;
-      const int lo = span_lo[i];
-      const int hi = span_hi[i];
-      const R *src = src_base + span_base[i] + s0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const bool valid = s0 + q >= lo && s0 + q < hi;
-        cp_async<sizeof(R)>(rb + i * LT + j0 + q, valid ? src + q : src_base, valid);
-      }
-    }
-  };
-  issue(0, raw[0]);
-  cp_async_commit();
-  for (int t = 0; t < job.T; ++t) {
-    if (t + 1 < job.T) issue(t + 1, raw[(t + 1) & 1]);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    const R *rb = raw[t & 1];
-    for (int idx = threadIdx.x; idx < NB * M; idx += kThreads) {
-      const int i = idx / M;
-      const int m = idx - i * M;
-      const int j = 2 * m;
-      R v0 = (R)0, v1 = (R)0;
-      if (j < LT) {
-        v0 = (rb[i * LT + j] * scale[i]) * taper[j];
-        v1 = (rb[i * LT + j + 1] * scale[i]) * taper[j + 1];
-      }
-      line[i * LS + m] = cmake<C>(v0, v1);
-    }
-    __syncthreads();
-    lines_fourstep<R, M1, M2, false>(line, NB, LS, twM);
-    // split: X_k = (Z_k + conj Z_{M-k}) / 2 - i e^{-2 pi i k / Pt} (Z_k - conj Z_{M-k}) / 2
-    C *zt = job.z + (long)t * F * ntr + t0;
-    for (int idx = threadIdx.x; idx < NB * F; idx += kThreads) {
-      const int f = idx / NB;
-      const int i = idx - f * NB;
-      if (i < nb) {
-        const C *b = line + i * LS;
-        const C zk = b[fourstep_pos<M1, M2>(f % M)];
-        const C zm = b[fourstep_pos<M1, M2>((M - f) % M)];
-        const C zc = cmake<C>(zm.x, -zm.y);
-        const C e = cmake<C>((R)0.5 * (zk.x + zc.x), (R)0.5 * (zk.y + zc.y));
-        const C o = cmake<C>((R)0.5 * (zk.y - zc.y), (R)-0.5 * (zk.x - zc.x));
-        C x = cadd(e, cmul(tw_at<false>(tw2M, f), o));
-        if (f >= 1 && f <= M - 1) x = cmake<C>(x.x * (R)2, x.y * (R)2);
-        zt[f * ntr + i] = x;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// ------------------------------------------------------------ fused time kernels
-
-// Hermitian combine of the c2r input (bins X of one trace, F = M + 1):
-// Z_k = (X_k + conj X_{M-k}) + i e^{+2 pi i k / Pt} (X_k - conj X_{M-k}),
-// the imaginary parts of X_0 and X_M dropped (c2r ignores them).
-template <typename R, int M>
-__device__ __forceinline__ Cx<R> combine_bin(const Cx<R> *x, int k, const Cx<R> *tw2M) {
-  using C = Cx<R>;
-  C a = x[k];
-  C b = x[M - k];
-  if (k == 0) {
-    a.y = (R)0;
-    b.y = (R)0;
-  }
-  const C bc = cmake<C>(b.x, -b.y);
-  const C e = cadd(a, bc);
-  const C d = csub(a, bc);
-  const C o = cmul(d, tw_at<true>(tw2M, k));
-  return cmake<C>(e.x - o.y, e.y + o.x);
-}
-
-// Forward time axis, fused: as time_fwd_fast, but the Hermitian combine is
-// done while loading the first four-step pass, and the second pass keeps
-// its outputs in registers: thread (trace i, k1) holds the samples
-// j = 2 (k1 + M1 k2) + c, and as H / 2 = 2 M / 5 = 4 M1 (M2 = 10), the
-// samples j < H (k2 < 4) and their successors j + H (k2 + 4) belong to the
-// same thread, so taper, overlap-add and the one-hop carry stay in
-// registers.  Two barriers per time window.  NB = 256 / M1 traces per block;
-// M2 = 10.  Bins lines LSB apart, work groups M2 + 1 apart within lines LSW
-// apart (both 10 mod 16, so the passes hit distinct banks).
-template <typename R, int M1, int M2, int LSB, int LSW, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB)
-    time_fwd_fused(const TimeJob<R> *__restrict__ jobs, const int *__restrict__ cta_job,
-                   const int *__restrict__ cta_trace0) {
-  using C = Cx<R>;
-  constexpr int M = M1 * M2;
-  constexpr int F = M + 1;
-  constexpr int H = 4 * M / 5;
-  constexpr int NB = kThreads / M1;
-  constexpr int G = M2 + 1;  // work group stride
-  static_assert(M2 == 10 && NB * M1 == kThreads, "fused time kernel shape");
-  static_assert(LSB >= F && LSW >= M1 * G, "line strides");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ C twM[M];
-  __shared__ C tw2M[2 * M];
-  load_twiddles<R, M>(twM);
-  load_twiddles<R, 2 * M>(tw2M);
-  const TimeJob<R> job = jobs[cta_job[blockIdx.x]];
-  const int t0 = cta_trace0[blockIdx.x];
-  const int nb = min(NB, job.n_traces - t0);
-  const long ntr = job.n_traces;
-  C *stage[2] = {reinterpret_cast<C *>(smem_raw), reinterpret_cast<C *>(smem_raw) + NB * LSB};
-  C *work = stage[1] + NB * LSB;
-  // this thread's trace and second-pass line, fixed over the time windows
-  const int ti = threadIdx.x / M1;
-  const int k1 = threadIdx.x - ti * M1;
-  const bool live = ti < nb;
-  const R sc = live ? job.space_scale[t0 + ti] : (R)0;
-  R tap[8][2];  // tapers of the samples j = 2 (k1 + M1 k2) + c, k2 < 8
-#pragma unroll
-  for (int k2 = 0; k2 < 8; ++k2)
-#pragma unroll
-    for (int c = 0; c < 2; ++c) tap[k2][c] = job.time_taper[2 * (k1 + M1 * k2) + c];
-  R carry[4][2];
-#pragma unroll
-  for (int k2 = 0; k2 < 4; ++k2) carry[k2][0] = carry[k2][1] = (R)0;
-  R *yrow = job.y + (long)(t0 + (live ? ti : 0)) * job.C;
-  auto issue = [&](int t, C *buf) {
-    const C *zt = job.z + (long)t * F * ntr + t0;
-    for (int idx = threadIdx.x; idx < NB * F; idx += kThreads) {
-      const int f = idx / NB;
-      const int i = idx - f * NB;
-      if (i < nb) cp_async<sizeof(C)>(buf + i * LSB + f, zt + f * ntr + i);
-    }
-  };
-  issue(0, stage[0]);
-  cp_async_commit();
-  for (int t = 0; t < job.T; ++t) {
-    if (t + 1 < job.T) issue(t + 1, stage[(t + 1) & 1]);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    const C *bins = stage[t & 1];
-    // first pass: lines (trace i, n2) over n1, combined bins as input
-    for (int it = threadIdx.x; it < NB * M2; it += kThreads) {
-      const int i = it / M2;
-      const int n2 = it - i * M2;
-      C v[M1];
-      if (i < nb) {
-#pragma unroll
-        for (int n1 = 0; n1 < M1; ++n1) v[n1] = combine_bin<R, M>(bins + i * LSB, M2 * n1 + n2, tw2M);
-      } else {
-#pragma unroll
-        for (int n1 = 0; n1 < M1; ++n1) v[n1] = cmake<C>((R)0, (R)0);
-      }
-      dft<R, M1, true>(v);
-      C *w = work + i * LSW + n2;
-#pragma unroll
-      for (int q = 0; q < M1; ++q)
-        w[G * q] = (q == 0) ? v[0] : cmul(v[q], tw_at<true>(twM, (n2 * q) % M));
-    }
-    __syncthreads();
-    // second pass: line k1 of trace ti; outputs X[k1 + M1 k2] = samples
-    // 2 (k1 + M1 k2) + {0, 1}
-    C v[M2];
-    const C *w = work + ti * LSW + G * k1;
-#pragma unroll
-    for (int n2 = 0; n2 < M2; ++n2) v[n2] = w[n2];
-    dft<R, M2, true>(v);
-    if (live) {
-      R *yt = yrow + t * H;
-#pragma unroll
-      for (int k2 = 0; k2 < 4; ++k2) {
-        const int j = 2 * (k1 + M1 * k2);
-        yt[j] = carry[k2][0] + (v[k2].x * sc) * tap[k2][0];
-        yt[j + 1] = carry[k2][1] + (v[k2].y * sc) * tap[k2][1];
-      }
-#pragma unroll
-      for (int k2 = 0; k2 < 4; ++k2) {
-        carry[k2][0] = (v[k2 + 4].x * sc) * tap[k2 + 4][0];
-        carry[k2][1] = (v[k2 + 4].y * sc) * tap[k2 + 4][1];
-      }
-    }
-  }
-  // last half window, then zeros up to C
-  if (live) {
-    R *yt = yrow + job.T * H;
-#pragma unroll
-    for (int k2 = 0; k2 < 4; ++k2) {
-      const int j = 2 * (k1 + M1 * k2);
-      yt[j] = carry[k2][0];
-      yt[j + 1] = carry[k2][1];
-    }
-  }
-  const int tail = job.C - (job.T + 1) * H;
-  for (int idx = threadIdx.x; idx < nb * tail; idx += kThreads) {
-    const int i = idx / tail;
-    const int j = idx - i * tail;
-    job.y[(long)(t0 + i) * job.C + (job.T + 1) * H + j] = (R)0;
-  }
-}
-
-// Adjoint time axis, fused: as time_adj_fast, but the scaling, tapering and
-// packing of the raw samples is done while loading the first four-step
-// pass, and the second pass writes its outputs back into its own group of
-// the work buffer (no second buffer).  Three barriers per time window.
-template <typename R, int M1, int M2, int LSW, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB)
-    time_adj_fused(const TimeJob<R> *__restrict__ jobs, const int *__restrict__ cta_job,
-                   const int *__restrict__ cta_trace0, const R *__restrict__ record,
-                   int from_record) {
-  using C = Cx<R>;
-  constexpr int M = M1 * M2;
-  constexpr int F = M + 1;
-  constexpr int H = 4 * M / 5;
-  constexpr int LT = 2 * H;
-  constexpr int NB = kThreads / M1;
-  constexpr int G = M2 + 1;
-  // raw sample rows padded to 20 mod 32 floats: the first pass reads sample
-  // pairs as 8-byte loads, and a half-warp's pairs then fall in distinct
-  // banks
-  constexpr int LTP = LT + ((20 - LT % 32) + 32) % 32;
-  static_assert(M2 == 10 && NB * M1 == kThreads, "fused time kernel shape");
-  static_assert(LSW >= M1 * G, "line stride");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ C twM[M];
-  __shared__ C tw2M[2 * M];
-  __shared__ long span_base[NB];
-  __shared__ int span_lo[NB], span_hi[NB];
-  __shared__ R scale[NB];
-  __shared__ R taper[LT];
-  load_twiddles<R, M>(twM);
-  load_twiddles<R, 2 * M>(tw2M);
-  const TimeJob<R> job = jobs[cta_job[blockIdx.x]];
-  const int t0 = cta_trace0[blockIdx.x];
-  const int nb = min(NB, job.n_traces - t0);
-  const long ntr = job.n_traces;
-  for (int j = threadIdx.x; j < LT; j += kThreads) taper[j] = job.time_taper[j];
-  for (int i = threadIdx.x; i < NB; i += kThreads) {
-    const int tr = t0 + i;
-    span_lo[i] = 0;
-    span_hi[i] = 0;
-    span_base[i] = 0;
-    scale[i] = (R)0;
-    if (i >= nb) continue;
-    scale[i] = job.space_scale[tr];
-    if (from_record) {
-      const long rec = job.blend_rec[tr];
-      const int ts = job.blend_ts[tr];
-      span_base[i] = rec - ts;
-      span_lo[i] = rec >= 0 ? ts : 0;
-      span_hi[i] = rec >= 0 ? ts + job.blend_n[tr] : 0;
-    } else {
-      span_base[i] = (long)tr * job.C;
-      span_hi[i] = job.C;
-    }
-  }
-  __syncthreads();
-  const R *src_base = from_record ? record : job.y;
-  C *work = reinterpret_cast<C *>(smem_raw);
-  R *raw[2] = {reinterpret_cast<R *>(work + NB * LSW),
-               reinterpret_cast<R *>(work + NB * LSW) + NB * LTP};
-  auto issue = [&](int t, R *rb) {
-    for (int g = threadIdx.x; g < NB * (LT / 4); g += kThreads) {
-      const int i = g / (LT / 4);
-      const int j0 = 4 * (g - i * (LT / 4));
-      const int s0 = t * H + j0;
-      const int lo = span_lo[i];
-      const int hi = span_hi[i];
-      const R *src = src_base + span_base[i] + s0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const bool valid = s0 + q >= lo && s0 + q < hi;
-        cp_async<sizeof(R)>(rb + i * LTP + j0 + q, valid ? src + q : src_base, valid);
-      }
-    }
-  };
-  const int ti = threadIdx.x / M1;
-  const int k1 = threadIdx.x - ti * M1;
-  issue(0, raw[0]);
-  cp_async_commit();
-  for (int t = 0; t < job.T; ++t) {
-    if (t + 1 < job.T) issue(t + 1, raw[(t + 1) & 1]);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    const R *rb = raw[t & 1];
-    // first pass: packed, tapered samples (2 m, 2 m + 1) as input
-    for (int it = threadIdx.x; it < NB * M2; it += kThreads) {
-      const int i = it / M2;
-      const int n2 = it - i * M2;
-      const R sc = scale[i];
-      C v[M1];
-#pragma unroll
-      for (int n1 = 0; n1 < M1; ++n1) {
-        const int j = 2 * (M2 * n1 + n2);
-        R v0 = (R)0, v1 = (R)0;
-        if (j < LT) {
-          const Cx<R> pr = *reinterpret_cast<const Cx<R> *>(rb + i * LTP + j);
-          v0 = (pr.x * sc) * taper[j];
-          v1 = (pr.y * sc) * taper[j + 1];
-        }
-        v[n1] = cmake<C>(v0, v1);
-      }
-      dft<R, M1, false>(v);
-      C *w = work + i * LSW + n2;
-#pragma unroll
-      for (int q = 0; q < M1; ++q)
-        w[G * q] = (q == 0) ? v[0] : cmul(v[q], tw_at<false>(twM, (n2 * q) % M));
-    }
-    __syncthreads();
-    {  // second pass, in place in this thread's group: Z[k1 + M1 k2]
-      C v[M2];
-      C *w = work + ti * LSW + G * k1;
-#pragma unroll
-      for (int n2 = 0; n2 < M2; ++n2) v[n2] = w[n2];
-      dft<R, M2, false>(v);
-#pragma unroll
-      for (int k2 = 0; k2 < M2; ++k2) w[k2] = v[k2];
-    }
-    __syncthreads();
-    // split: X_k = (Z_k + conj Z_{M-k}) / 2 - i e^{-2 pi i k / Pt} (Z_k - conj Z_{M-k}) / 2
-    C *zt = job.z + (long)t * F * ntr + t0;
-    for (int idx = threadIdx.x; idx < NB * F; idx += kThreads) {
-      const int f = idx / NB;
-      const int i = idx - f * NB;
-      if (i < nb) {
-        const C *b = work + i * LSW;
-        const int fa = f % M;
-        const int fb = (M - f) % M;
-        const C zk = b[G * (fa % M1) + fa / M1];
-        const C zm = b[G * (fb % M1) + fb / M1];
-        const C zc = cmake<C>(zm.x, -zm.y);
-        const C e = cmake<C>((R)0.5 * (zk.x + zc.x), (R)0.5 * (zk.y + zc.y));
-        const C o = cmake<C>((R)0.5 * (zk.y - zc.y), (R)-0.5 * (zk.x - zc.x));
-        C x = cadd(e, cmul(tw_at<false>(tw2M, f), o));
-        if (f >= 1 && f <= M - 1) x = cmake<C>(x.x * (R)2, x.y * (R)2);
-        zt[f * ntr + i] = x;
-      }
-    }
   }
 }
 
