@@ -97,6 +97,16 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
+// Brings n bytes of global memory into L2 (whole 16-byte pieces of it),
+// issued by the calling thread alone.
+__device__ __forceinline__ void prefetch_l2(const void *p, long n) {
+  const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15;
+  const long m = (reinterpret_cast<uintptr_t>(p) + n - a) & ~15L;
+  if (m > 0)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)m)
+                 : "memory");
+}
+
 // ------------------------------------------------------------ register DFTs
 
 template <bool INV, typename C>
@@ -524,6 +534,8 @@ __global__ void __launch_bounds__(NT, MINB) space_fwd_fast(PlaneBatches<R> batch
       cp_async_wait<0>();
     }
     __syncthreads();
+    if (STAGES == 1 && threadIdx.x == 0 && nxt.count > 0)
+      prefetch_l2(nxt.src, (long)nxt.count * S::dense_P * (long)sizeof(C));
     C *buf = stage[STAGES == 2 ? (k & 1) : 0];
     const int np = cur.count;
     space_axes<R, D, P0, P1, P2, NT, NP, true>(buf, np);
@@ -1016,7 +1028,11 @@ __global__ void __launch_bounds__(NT, MINB)
                      S::S1, S::S0, 1, S::L0, P0>(stg, work, np);
     }
     __syncthreads();
-    if (nxt.count > 0) copy_in(stg, nxt.src, nxt.count * S::dense_L);
+    if (nxt.count > 0) {
+      copy_in(stg, nxt.src, nxt.count * S::dense_L);
+      if (!XS && need_x && threadIdx.x == 0)
+        prefetch_l2(nxt.dst, (long)nxt.count * S::dense_P * (long)sizeof(C));
+    }
     cp_async_commit();
     const R step = multi ? step_dev[cur.pid] : step_arg;
     const R lamb = lamb_dev != nullptr ? lamb_dev[multi ? cur.pid : 0] : lamb_arg;

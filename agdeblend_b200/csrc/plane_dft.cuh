@@ -341,16 +341,6 @@ __device__ __forceinline__ void dft_rows_in_place(Cx<R> *rows, int rs, int n,
   }
 }
 
-// Brings n bytes of global memory into L2 (whole 16-byte pieces of it),
-// issued by the calling thread alone.
-__device__ __forceinline__ void prefetch_l2(const void *p, long n) {
-  const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15;
-  const long m = (reinterpret_cast<uintptr_t>(p) + n - a) & ~15L;
-  if (m > 0)
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)m)
-                 : "memory");
-}
-
 // Finished rows of shared memory (stride rs) to n rows of n_out values at
 // dst, with the update (epilogues as axis_pass); returns the largest |x|^2
 // of kUpdateMax.  A fixed thread -> (row, column) map (no index division),
