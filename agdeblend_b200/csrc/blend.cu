@@ -165,9 +165,8 @@ extern "C" int agd_blend(int n_patches, int const *n_traces, int const *n_times,
   if (n_chunk > 0) {
     agd::blend_gather<real><<<(unsigned)n_chunk, agd::kThreads, 0, s>>>(
         (const agd::Contrib *)d_flat.p, (const long *)d_ptr.p, agd::BlendTables::kChunk, R,
-        (const real *)d_in.p, (real *)d_rec.p, bt.mode, (const uint8_t *)d_mute.p, nullptr,
-        (const real *)d_taper.p,
-        (int)taper.size(), nullptr);
+        (const real *)d_in.p, (real *)d_rec.p, bt.mode, (const uint8_t *)d_mute.p,
+        (const real *)d_taper.p, (int)taper.size());
     BCK(cudaGetLastError());
   }
   if (n_out_tr) {

@@ -184,8 +184,8 @@ extern "C" int agd_blend_device_noalloc(
         reinterpret_cast<const agd::Contrib *>(base + at_flat),
         reinterpret_cast<const long *>(base + at_ptr), agd::BlendTables::kChunk, R, data_dev,
         record, bt.mode,
-        reinterpret_cast<const uint8_t *>(base + at_mute), nullptr,
-        reinterpret_cast<const real *>(base + at_taper), (int)taper.size(), nullptr);
+        reinterpret_cast<const uint8_t *>(base + at_mute),
+        reinterpret_cast<const real *>(base + at_taper), (int)taper.size());
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && n_out > 0) {

@@ -218,8 +218,7 @@ int agd_gpu_forward(agd_gpu_problem *pb, AGD_TYPE const *model, AGD_TYPE *record
     agd::EngineR &e = *pb->eng;
     e.model_from_ref(model);
     e.forward_traces();
-    e.launch_gather(e.g_fwd, e.Y.get(), e.rec_r.get(), agd::kGatherSum, true, nullptr, nullptr,
-                    0, nullptr);
+    e.launch_record_gather(e.rec_r.get(), true, nullptr, nullptr);
     if (e.plan.record_size)
       agd::CK(cudaMemcpyAsync(record, e.rec_r.get(), e.rec_r.bytes(), cudaMemcpyDeviceToHost,
                               e.stream));

@@ -151,7 +151,15 @@ class Engine {
   int n_sm = 148;
   int sm_smem = 233472;      // shared memory per SM (bytes)
   int block_reserved = 1024;  // shared memory the system reserves per block
-  GatherLaunch g_fwd, g_input;
+  GatherLaunch g_input;
+  // the forward operator's gather: chunk-local runs
+  struct RecordLaunch {
+    DevArray<GatherRun> runs;
+    DevArray<long> chunk_ptr;
+    int n_chunk = 0;
+    long n_contrib = 0;
+  };
+  RecordLaunch g_fwd;
   std::vector<long> trace_off;   // per window, in reals
   std::vector<long> patch_off;   // per patch, in reals
   long n_wtraces = 0;
@@ -208,7 +216,7 @@ class Engine {
 
   size_t device_bytes() const {
     return X.bytes() + S0.bytes() + S1.bytes() + G.bytes() + Y.bytes() + rec_d.bytes() +
-           rec_r.bytes() + data_dev.bytes() + mute.bytes() + g_fwd.contrib.bytes() +
+           rec_r.bytes() + data_dev.bytes() + mute.bytes() + g_fwd.runs.bytes() +
            g_input.contrib.bytes();
   }
 
@@ -1545,6 +1553,28 @@ class Engine {
     G.n_contrib = (long)list.size();
   }
 
+  // Runs of the forward gather, each contribution cut at the record's chunks.
+  void make_record_gather(const std::vector<Contrib> &list) {
+    RecordLaunch &G = g_fwd;
+    constexpr long chunk = kRecordChunk;
+    G.n_chunk = (int)((plan.record_size + chunk - 1) / chunk);
+    std::vector<long> count(G.n_chunk + 1, 0);
+    for (const Contrib &c : list)
+      for (long k = c.rec / chunk; c.n > 0 && k <= (c.rec + c.n - 1) / chunk; ++k) count[k + 1]++;
+    for (int k = 0; k < G.n_chunk; ++k) count[k + 1] += count[k];
+    std::vector<GatherRun> flat(count[G.n_chunk]);
+    std::vector<long> fill(count.begin(), count.end() - 1);
+    for (const Contrib &c : list)
+      for (long k = c.rec / chunk; c.n > 0 && k <= (c.rec + c.n - 1) / chunk; ++k) {
+        const long c0 = k * chunk;
+        flat[fill[k]++] = GatherRun{c.src + (c0 - c.rec), (int)std::max(0L, c.rec - c0),
+                                    (int)std::min(chunk, c.rec + c.n - c0)};
+      }
+    G.runs.upload(flat, stream);
+    G.chunk_ptr.upload(count, stream);
+    G.n_contrib = (long)list.size();
+  }
+
   void build() {
     setup_mark("", true);
     const long M = plan.model_size;
@@ -1754,7 +1784,7 @@ class Engine {
           list.push_back(c);
         }
       }
-      make_gather(g_fwd, list, plan.record_size);
+      make_record_gather(list);
     }
 
     // ---- input blend and output gather tables (patch traces)
@@ -1856,12 +1886,20 @@ class Engine {
     CK(cudaGetLastError());
   }
 
-  void launch_gather(const GatherLaunch &Gl, const R *src, R *out, int mode, bool use_mute,
-                     const R *d, const R *taper, int taper_len, double *sumsq) {
-    if (Gl.n_chunk == 0) return;
-    blend_gather<R><<<Gl.n_chunk, kThreads, 0, stream>>>(
-        Gl.contrib.get(), Gl.chunk_ptr.get(), Gl.chunk, plan.record_size, src, out, mode,
-        use_mute ? mute.get() : nullptr, d, taper, taper_len, sumsq);
+  void launch_input_gather(const R *src, R *out) {
+    if (g_input.n_chunk == 0) return;
+    blend_gather<R><<<g_input.n_chunk, kThreads, 0, stream>>>(
+        g_input.contrib.get(), g_input.chunk_ptr.get(), g_input.chunk, plan.record_size, src, out,
+        kGatherMean, mute.get(), nullptr, 0);
+    CK(cudaGetLastError());
+  }
+
+  // record <- sum of the window traces (muted with use_mute), minus d
+  void launch_record_gather(R *out, bool use_mute, const R *d, double *sumsq) {
+    if (g_fwd.n_chunk == 0) return;
+    record_gather<R><<<g_fwd.n_chunk, kThreads, 0, stream>>>(
+        g_fwd.runs.get(), g_fwd.chunk_ptr.get(), plan.record_size, Y.get(), out,
+        use_mute ? mute.get() : nullptr, d, sumsq);
     CK(cudaGetLastError());
   }
 
@@ -2112,8 +2150,7 @@ class Engine {
       CK(cudaMemsetAsync(dscalar.get(), 0, sizeof(double), stream));
       ss = dscalar.get();
     }
-    launch_gather(g_fwd, Y.get(), rec_r.get(), kGatherResidual, true, rec_d.get(), nullptr, 0,
-                  ss);
+    launch_record_gather(rec_r.get(), true, rec_d.get(), ss);
   }
 
   double read_dscalar() {
@@ -2162,7 +2199,7 @@ class Engine {
           Y.get(), space_fold.get(), wt_dst.get(), wt_C.get(), n_wtraces);
       CK(cudaGetLastError());
     }
-    launch_gather(g_fwd, Y.get(), rec_r.get(), kGatherSum, false, nullptr, nullptr, 0, nullptr);
+    launch_record_gather(rec_r.get(), false, nullptr, nullptr);
     if (multi) {  // one maximum per problem, over its record range
       const int np = plan.n_problems;
       std::vector<R> fac(np, (R)1);
@@ -2234,8 +2271,7 @@ class Engine {
       }
       set_input_gather(list);
     }
-    launch_gather(g_input, data_dev.get(), rec_d.get(), kGatherMean, true, nullptr, nullptr, 0,
-                  nullptr);
+    launch_input_gather(data_dev.get(), rec_d.get());
   }
 
   void output() {

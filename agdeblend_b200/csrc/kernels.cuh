@@ -80,7 +80,6 @@ enum GatherMode : int {
   kGatherSum = 0,
   kGatherMean = 1,
   kGatherOverwrite = 2,
-  kGatherResidual = 3,  // out = mask ? 0 : sum - d
 };
 
 // ------------------------------------------------------------ helpers
@@ -452,8 +451,8 @@ template <typename R>
 __global__ void __launch_bounds__(kThreads)
     blend_gather(const Contrib *__restrict__ contrib, const long *__restrict__ chunk_ptr,
                  int chunk, long record_size, const R *__restrict__ src, R *out,
-                 int mode, const uint8_t *__restrict__ mute, const R *__restrict__ d,
-                 const R *__restrict__ taper, int taper_len, double *sumsq) {
+                 int mode, const uint8_t *__restrict__ mute, const R *__restrict__ taper,
+                 int taper_len) {
   __shared__ Contrib tile[kGatherTile];
   const long c0 = (long)blockIdx.x * chunk;
   const long b0 = chunk_ptr[blockIdx.x];
@@ -539,7 +538,6 @@ __global__ void __launch_bounds__(kThreads)
       cnt[q] = w_sum;
     }
   }
-  double local = 0.0;
 #pragma unroll
   for (int q = 0; q < kGatherSpt; ++q) {
     const int k = threadIdx.x + q * blockDim.x;
@@ -547,14 +545,79 @@ __global__ void __launch_bounds__(kThreads)
     if (k >= chunk || s >= record_size) continue;
     R a = acc[q];
     if (mode == kGatherMean && cnt[q] > (R)0) a /= cnt[q];
-    if (mode == kGatherResidual) a = a - d[s];
     if (mute != nullptr && mute[s]) a = (R)0;
     out[s] = a;
-    local += (double)a * (double)a;
   }
+}
+
+// The forward operator's gather: record[s] = sum of the window traces'
+// samples at s, in list order (the serial reference's window-then-trace
+// order), minus d with the residual, zero where muted.  Block b owns the
+// kRecordChunk samples from b * kRecordChunk on.  Bound by the reads of the
+// traces; a run is described by chunk-local numbers (16 bytes, one shared
+// load: the index of the chunk's first sample and the covered range), so a
+// sample costs two compares and one load, and the loads of eight runs are in
+// flight per thread.  Survey of 50,176 traces (257 MB): 123 us with runs in
+// record coordinates and four in flight, 56 us (40 us at the copy
+// bandwidth).
+struct GatherRun {
+  long base;   // source index of the chunk's sample 0 (outside the source where not covered)
+  int lo, hi;  // covered samples of the chunk
+};
+
+constexpr int kRecordChunk = 2 * kThreads;
+constexpr int kRunsInFlight = 8;
+
+template <typename R>
+__global__ void __launch_bounds__(kThreads)
+    record_gather(const GatherRun *__restrict__ runs, const long *__restrict__ chunk_ptr,
+                  long record_size, const R *__restrict__ src, R *__restrict__ out,
+                  const uint8_t *__restrict__ mute, const R *__restrict__ d, double *sumsq) {
+  __shared__ GatherRun tile[kGatherTile];
+  const long s0 = (long)blockIdx.x * kRecordChunk + threadIdx.x;
+  const long b0 = chunk_ptr[blockIdx.x];
+  const long b1 = chunk_ptr[blockIdx.x + 1];
+  const int k0 = threadIdx.x, k1 = threadIdx.x + kThreads;
+  const bool on0 = s0 < record_size, on1 = s0 + kThreads < record_size;
+  const R d0 = d != nullptr && on0 ? d[s0] : (R)0;
+  const R d1 = d != nullptr && on1 ? d[s0 + kThreads] : (R)0;
+  const bool m0 = mute != nullptr && on0 && mute[s0];
+  const bool m1 = mute != nullptr && on1 && mute[s0 + kThreads];
+  R a0 = (R)0, a1 = (R)0;
+  for (long base = b0; base < b1; base += kGatherTile) {
+    const int n = (int)min((long)kGatherTile, b1 - base);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kThreads) tile[i] = runs[base + i];
+    __syncthreads();
+    int c = 0;
+    for (; c + kRunsInFlight <= n; c += kRunsInFlight) {
+      R v0[kRunsInFlight], v1[kRunsInFlight];
+#pragma unroll
+      for (int u = 0; u < kRunsInFlight; ++u) {
+        const GatherRun r = tile[c + u];
+        v0[u] = k0 >= r.lo && k0 < r.hi ? src[r.base + k0] : (R)0;
+        v1[u] = k1 >= r.lo && k1 < r.hi ? src[r.base + k1] : (R)0;
+      }
+#pragma unroll
+      for (int u = 0; u < kRunsInFlight; ++u) {  // adding 0 changes no sum
+        a0 += v0[u];
+        a1 += v1[u];
+      }
+    }
+    for (; c < n; ++c) {
+      const GatherRun r = tile[c];
+      if (k0 >= r.lo && k0 < r.hi) a0 += src[r.base + k0];
+      if (k1 >= r.lo && k1 < r.hi) a1 += src[r.base + k1];
+    }
+  }
+  a0 = m0 ? (R)0 : a0 - d0;
+  a1 = m1 ? (R)0 : a1 - d1;
+  if (on0) out[s0] = a0;
+  if (on1) out[s0 + kThreads] = a1;
   if (sumsq != nullptr) {
     __shared__ double red[32];
-    const double t = block_sum(local, red);
+    const double t = block_sum((on0 ? (double)a0 * (double)a0 : 0.0) +
+                                   (on1 ? (double)a1 * (double)a1 : 0.0), red);
     if (threadIdx.x == 0) atomicAdd(sumsq, t);
   }
 }
