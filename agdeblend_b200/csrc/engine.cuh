@@ -406,31 +406,47 @@ class Engine {
     return (size_t)n_max * sizeof(C) <= (size_t)smem_max;
   }
 
-  // Spectra of the wavelet sources: the plan's where the transform has the
-  // trace's length (and for the generic kernel), the padded ones made on the
-  // device from it where it is longer.
+  // Spectra of the wavelet sources.  Generic kernel (no shapes): the plan's
+  // half spectra.  Prime-factor kernel: whole spectra in the dense frequency
+  // order of the source's transform, the plan's where the transform has the
+  // trace's length, the padded ones made from it on the device where it is
+  // longer.
   void upload_spectra(const std::vector<PfaShape> &shapes) {
-    std::map<int, int> n_of;  // trace length -> transform length
-    for (size_t w = 0; w < shapes.size(); ++w) n_of[plan.windows[w].C] = shapes[w].N;
     std::vector<C> sp;
     std::vector<long> so;
-    long c_max = 0;
-    auto length = [&](size_t i) {
-      const auto it = n_of.find(plan.wavelet_n[i]);
-      return it == n_of.end() ? plan.wavelet_n[i] : it->second;
+    auto put = [](C &c, std::complex<double> v) {
+      c.x = (R)v.real();
+      c.y = (R)v.imag();
     };
+    if (shapes.empty()) {
+      for (const auto &s : plan.spectra) {
+        so.push_back((long)sp.size());
+        for (const auto &v : s) put((sp.emplace_back(), sp.back()), v);
+      }
+      spectra.upload(sp, stream);
+      spec_off.upload(so, stream);
+      return;
+    }
+    std::map<int, const PfaShape *> shape_of;  // by trace length
+    for (size_t w = 0; w < shapes.size(); ++w) shape_of[plan.windows[w].C] = &shapes[w];
+    std::vector<unsigned short> map;
+    long c_max = 0;
     for (size_t i = 0; i < plan.spectra.size(); ++i) {
-      so.push_back((long)sp.size());
-      if (length(i) != plan.wavelet_n[i]) {
-        sp.resize(sp.size() + length(i) / 2 + 1);
+      const PfaShape &sh = *shape_of.at(plan.wavelet_n[i]);
+      const int N = sh.N;
+      const long o = (long)sp.size();
+      so.push_back(o);
+      sp.resize(o + N);
+      if (N != plan.wavelet_n[i]) {
         c_max = std::max(c_max, (long)plan.wavelet_n[i]);
         continue;
       }
-      for (const auto &v : plan.spectra[i]) {
-        C c;
-        c.x = (R)v.real();
-        c.y = (R)v.imag();
-        sp.push_back(c);
+      map.clear();
+      pfa_tables(sh, map);
+      const unsigned short *kpos = map.data() + N;
+      for (int k = 0; k <= N / 2; ++k) {
+        put(sp[o + kpos[k]], plan.spectra[i][k]);
+        if (k > 0 && 2 * k != N) put(sp[o + kpos[N - k]], std::conj(plan.spectra[i][k]));
       }
     }
     spectra.upload(sp, stream);
@@ -438,20 +454,25 @@ class Engine {
     if (c_max == 0) return;
     DevArray<double2> half;
     DevArray<double> taps;
+    DevArray<unsigned short> kpos;
     half.alloc(c_max / 2 + 1);
     taps.alloc(c_max);
     for (size_t i = 0; i < plan.spectra.size(); ++i) {
-      const int n = plan.wavelet_n[i], N = length(i);
-      if (N == n) continue;
+      const int n = plan.wavelet_n[i];
+      const PfaShape &sh = *shape_of.at(n);
+      if (sh.N == n) continue;
+      map.clear();
+      pfa_tables(sh, map);
+      kpos.upload(map, stream);
       CK(cudaMemcpyAsync(half.get(), plan.spectra[i].data(),
                          plan.spectra[i].size() * sizeof(double2), cudaMemcpyHostToDevice,
                          stream));
       wavelet_taps<<<n, kWavThreads, 0, stream>>>(half.get(), n, taps.get());
-      wavelet_pad_spectrum<R><<<N / 2 + 1, kWavThreads, 0, stream>>>(taps.get(), n, N,
-                                                                    spectra.get() + so[i]);
+      wavelet_pad_spectrum<R><<<sh.N / 2 + 1, kWavThreads, 0, stream>>>(
+          taps.get(), n, sh.N, kpos.get() + sh.N, spectra.get() + so[i]);
       CK(cudaGetLastError());
+      CK(cudaStreamSynchronize(stream));  // before the work arrays are reused or released
     }
-    CK(cudaStreamSynchronize(stream));  // before the work arrays are released
   }
 
   struct WaveletCand {

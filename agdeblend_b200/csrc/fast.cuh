@@ -160,8 +160,40 @@ __host__ __device__ constexpr int crt_index(int k1, int k2, int N1, int N2) {
   return k;
 }
 
-// Odd length N with a twiddle table: the outputs k and N-k share the sums
-// x_j + x_{N-j} (times cos) and x_j - x_{N-j} (times sin), so
+// cos and sin of 2 pi m / n at compile time (Taylor series about 0 of an
+// angle in [0, pi], in double precision), so that the register DFTs of odd
+// length have literal coefficients.
+constexpr double const_cos(int m, int n) {
+  const double x = 6.283185307179586476925286766559 * m / n;
+  double term = 1.0, sum = 1.0;
+  for (int i = 1; i < 24; ++i) {
+    term *= -x * x / ((2.0 * i - 1.0) * (2.0 * i));
+    sum += term;
+  }
+  return sum;
+}
+constexpr double const_sin(int m, int n) {
+  const double x = 6.283185307179586476925286766559 * m / n;
+  double term = x, sum = x;
+  for (int i = 1; i < 24; ++i) {
+    term *= -x * x / ((2.0 * i) * (2.0 * i + 1.0));
+    sum += term;
+  }
+  return sum;
+}
+template <typename R, int N>
+struct OddTable {  // m = 0 .. (N - 1) / 2
+  R c[(N + 1) / 2], s[(N + 1) / 2];
+  constexpr OddTable() : c(), s() {
+    for (int m = 0; m < (N + 1) / 2; ++m) {
+      c[m] = (R)const_cos(m, N);
+      s[m] = (R)const_sin(m, N);
+    }
+  }
+};
+
+// Odd length N: the outputs k and N-k share the sums x_j + x_{N-j} (times
+// cos) and x_j - x_{N-j} (times sin), so
 //   X_k = A_k -/+ i B_k,  X_{N-k} = A_k +/- i B_k   (forward / inverse),
 //   A_k = x_0 + sum_j (x_j + x_{N-j}) cos(2 pi j k / N),
 //   B_k = sum_j (x_j - x_{N-j}) sin(2 pi j k / N),   j = 1 .. (N-1)/2.
@@ -170,7 +202,7 @@ __device__ __forceinline__ void dft_odd(Cx<R> (&v)[N]) {
   using C = Cx<R>;
   static_assert(N % 2 == 1, "odd length");
   constexpr int H = (N - 1) / 2;
-  constexpr int off = tw_offset(N);
+  constexpr OddTable<R, N> tab{};
   C sum[H], dif[H];
   C tot = v[0];
 #pragma unroll
@@ -186,9 +218,11 @@ __device__ __forceinline__ void dft_odd(Cx<R> (&v)[N]) {
     C b = cmake<C>((R)0, (R)0);
 #pragma unroll
     for (int j = 1; j <= H; ++j) {
-      const C w = ctw<R>(off + (j * k) % N);  // (cos, -sin) of 2 pi j k / N
-      a = cfma(a, w.x, sum[j - 1]);
-      b = cfma(b, -w.y, dif[j - 1]);
+      const int m = j * k % N;
+      const R c = tab.c[m <= H ? m : N - m];
+      const R s = m <= H ? tab.s[m] : -tab.s[N - m];
+      a = cfma(a, c, sum[j - 1]);
+      b = cfma(b, s, dif[j - 1]);
     }
     v[k] = add_rot<INV>(a, b);
     v[N - k] = sub_rot<INV>(a, b);
@@ -319,7 +353,7 @@ __device__ __forceinline__ void dft(Cx<R> (&v)[N]) {
   } else if constexpr (small_split(N) != 0) {
     constexpr int N1 = small_split(N);
     dft_fourstep<R, N1, N / N1, INV>(v);
-  } else if constexpr (tw_offset(N) >= 0) {
+  } else if constexpr (N % 2 == 1) {
     dft_odd<R, N, INV>(v);
   } else {
     // prime length without a table: direct DFT (only small primes reach here)

@@ -20,9 +20,12 @@
 //    return the dense array to the sample layout, which the store reads
 //    back through qmap.  Consecutive samples lie sum_i g_i apart, an odd
 //    stride, so the copies in and out are free of bank conflicts.
-//  * between them, with Z' the product spectrum,
+//  * the outermost axis is the turning point: a thread transforms a line
+//    forward, multiplies it by the spectrum (kept in the dense frequency
+//    order) and transforms it back, where the traces of every pair of the
+//    block share a spectrum.  Otherwise, with Z' the product spectrum,
 //      Z'_k = ((Z_k + conj Z_{C-k}) S_a + (Z_k - conj Z_{C-k}) S_b) / 2,
-//    which is Z_k S when both traces use the same spectrum.  The real and
+//    in a step of its own (Z_k S when both use the same).  The real and
 //    imaginary parts of the inverse are the two filtered traces.  A trace
 //    without a spectrum (bare transform pair, i.e. C times the trace) stays
 //    out of the transform, as zeros, and is scaled when the pair is stored:
@@ -50,6 +53,7 @@ namespace agd {
 
 constexpr int kPfaMaxFactors = 4;
 constexpr int kWavThreads = 256;
+constexpr int kWavMaxPairs = 4;  // pairs of a block at most
 
 struct PfaShape {
   int N;                          // transform length
@@ -103,6 +107,38 @@ __device__ __forceinline__ void pfa_pass(Cx<R> *buf, int np, int N, int g, float
   }
 }
 
+// The turning point of the transform along the outermost axis, where the two
+// traces of every pair share a spectrum: the forward DFT of a line, its
+// products with the spectrum (stored in the dense frequency order, so that
+// the values of neighbouring lines lie side by side) and the inverse DFT,
+// without leaving the registers.  spec_of(pair): the pair's spectrum.
+template <typename R, int F, typename Spec>
+__device__ __forceinline__ void pfa_turn(Cx<R> *buf, int np, int N, int g, float inv_lines,
+                                         bool adjoint, Spec spec_of) {
+  using C = Cx<R>;
+  const int lines = N / F;  // = g
+  const int total = np * lines;
+  for (int idx = threadIdx.x; idx < total; idx += kWavThreads) {
+    const int pr = div_small(idx, inv_lines);
+    const int l = idx - pr * lines;
+    C *b = buf + pr * N + l;
+    const C *sp = spec_of(pr) + l;
+    C v[F];
+#pragma unroll
+    for (int m = 0; m < F; ++m) v[m] = b[m * g];
+    dft<R, F, false>(v);
+#pragma unroll
+    for (int m = 0; m < F; ++m) {
+      C w = __ldg(sp + m * g);
+      if (adjoint) w.y = -w.y;
+      v[m] = cmul(v[m], w);
+    }
+    dft<R, F, true>(v);
+#pragma unroll
+    for (int m = 0; m < F; ++m) b[m * g] = v[m];
+  }
+}
+
 // Factors above FMAX are compiled out (their register DFTs would raise the
 // register demand of every pass); the host picks an instantiation whose
 // FMAX covers the shape.
@@ -135,14 +171,33 @@ __device__ void pfa_pass_any(int F, Cx<R> *buf, int np, int N, int g, float inv_
 #undef AGD_PFA_CASE
 }
 
-// Spectrum value for frequency k of a real signal's length-N transform,
-// conjugated for the adjoint.
-template <typename R>
-__device__ __forceinline__ Cx<R> spectrum_at(const Cx<R> *sp, int k, int N, bool adjoint) {
-  using C = Cx<R>;
-  C w = k <= N / 2 ? sp[k] : cmake<C>(sp[N - k].x, -sp[N - k].y);
-  if (adjoint) w.y = -w.y;
-  return w;
+template <typename R, int FMAX, typename Spec>
+__device__ void pfa_turn_any(int F, Cx<R> *buf, int np, int N, int g, float inv_lines,
+                             bool adjoint, Spec spec_of) {
+#define AGD_PFA_CASE(n) \
+  case n: \
+    if constexpr (n <= FMAX) pfa_turn<R, n>(buf, np, N, g, inv_lines, adjoint, spec_of); \
+    break;
+  switch (F) {
+    AGD_PFA_CASE(2)
+    AGD_PFA_CASE(3)
+    AGD_PFA_CASE(4)
+    AGD_PFA_CASE(5)
+    AGD_PFA_CASE(7)
+    AGD_PFA_CASE(8)
+    AGD_PFA_CASE(9)
+    AGD_PFA_CASE(11)
+    AGD_PFA_CASE(13)
+    AGD_PFA_CASE(16)
+    AGD_PFA_CASE(17)
+    AGD_PFA_CASE(19)
+    AGD_PFA_CASE(23)
+    AGD_PFA_CASE(25)
+    AGD_PFA_CASE(27)
+    AGD_PFA_CASE(32)
+    default: break;
+  }
+#undef AGD_PFA_CASE
 }
 
 // Input sample t of trace tr: from the record through its blend coordinates
@@ -184,76 +239,95 @@ __global__ void __launch_bounds__(kWavThreads, MINB)
   // ---- load: trace a -> real part, trace b -> imaginary part, each sample
   // to its dense position; thread u copies half u & 1 of sample u >> 1, so a
   // warp fills 16 whole complex slots; every copy of the block in flight
-  // together
-  for (int pr = 0; pr < np; ++pr) {
-    const int ta = 2 * (pair0 + pr);
-    const int tb = ta + 1 < n_tr ? ta + 1 : -1;
-    const int mine = tb >= 0 ? ta + (threadIdx.x & 1) : ta;  // this thread's trace
-    R *b = reinterpret_cast<R *>(buf + pr * N) + (threadIdx.x & 1);
-    const bool live = (tb >= 0 || (threadIdx.x & 1) == 0) && job.src[mine] >= 0;
-    if (record != nullptr) {
-      const long r0 = job.blend_rec[mine];
-      const int s0 = job.blend_ts[mine];
-      const int n0 = live && r0 >= 0 ? job.blend_n[mine] : 0;
-      for (int t = threadIdx.x >> 1; t < N; t += kWavThreads / 2) {
-        const bool v = t >= s0 && t < s0 + n0;  // a span ends within the trace
-        cp_async<sizeof(R)>(b + 2 * __ldg(qmap + t), v ? record + r0 + (t - s0) : record, v);
+  // together, one position look-up for all pairs
+  {
+    const R *from[kWavMaxPairs];  // this thread's trace of each pair, sample 0
+    int lo[kWavMaxPairs], hi[kWavMaxPairs];
+#pragma unroll
+    for (int pr = 0; pr < kWavMaxPairs; ++pr) {
+      const int tr = 2 * (pair0 + pr) + (threadIdx.x & 1);
+      from[pr] = job.y;
+      lo[pr] = hi[pr] = 0;
+      if (pr >= np || tr >= n_tr || job.src[tr] < 0) continue;
+      if (record != nullptr) {
+        const long r0 = job.blend_rec[tr];
+        if (r0 < 0) continue;
+        lo[pr] = job.blend_ts[tr];
+        hi[pr] = lo[pr] + job.blend_n[tr];  // a span ends within the trace
+        from[pr] = record + r0 - lo[pr];
+      } else {
+        hi[pr] = Ct;
+        from[pr] = job.y + (long)tr * Ct;
       }
-    } else {
-      const R *y0 = job.y + (long)mine * Ct;
-      for (int t = threadIdx.x >> 1; t < N; t += kWavThreads / 2) {
-        const bool v = live && (!PADDED || t < Ct);
-        cp_async<sizeof(R)>(b + 2 * __ldg(qmap + t), v ? y0 + t : y0, v);
-      }
+    }
+    R *to = reinterpret_cast<R *>(buf) + (threadIdx.x & 1);
+    for (int t = threadIdx.x >> 1; t < N; t += kWavThreads / 2) {
+      R *slot = to + 2 * __ldg(qmap + t);
+#pragma unroll
+      for (int pr = 0; pr < kWavMaxPairs; ++pr)
+        if (pr < np) {
+          const bool v = t >= lo[pr] && t < hi[pr];
+          cp_async<sizeof(R)>(slot + 2 * pr * N, v ? from[pr] + t : job.y, v);
+        }
     }
   }
   cp_async_commit();
+  // spectrum of each pair's traces (a half without one holds zeros: any
+  // spectrum serves it)
+  __shared__ long at[kWavMaxPairs][2];
+  if (threadIdx.x < np) {
+    const int ta = 2 * (pair0 + threadIdx.x);
+    const int sa = job.src[ta];
+    const int sb = ta + 1 < n_tr ? job.src[ta + 1] : sa;
+    at[threadIdx.x][0] = sa >= 0 ? spec_off[sa] : sb >= 0 ? spec_off[sb] : 0;
+    at[threadIdx.x][1] = sb >= 0 ? spec_off[sb] : sa >= 0 ? spec_off[sa] : 0;
+  }
   cp_async_wait<0>();
   __syncthreads();
+  bool shared = true;
+  for (int pr = 0; pr < np; ++pr) shared = shared && at[pr][0] == at[pr][1];
 
-  for (int i = 0; i < sh.nf; ++i) {
+  const bool adjoint = direction < 0;
+  for (int i = sh.nf - 1; i > 0; --i) {
     pfa_pass_any<R, false, FMAX>(sh.f[i], buf, np, N, sh.g[i], sh.inv_g[i], sh.inv_lines[i]);
     __syncthreads();
   }
-
-  // ---- spectrum product (frequencies k and C - k together)
-  const bool adjoint = direction < 0;
-  const int half = N / 2 + 1;
-  for (int pr = 0; pr < np; ++pr) {
-    const int ta = 2 * (pair0 + pr);
-    // a half without a spectrum holds zeros: any spectrum serves it
-    const int sa = job.src[ta];
-    const int sb = ta + 1 < n_tr ? job.src[ta + 1] : sa;
-    const int wa = sa >= 0 ? sa : sb;
-    const int wb = sb >= 0 ? sb : sa;
-    if (wa < 0) continue;
-    const C *spa = spectra + spec_off[wa];
-    const C *spb = spectra + spec_off[wb];
-    C *b = buf + pr * N;
-    for (int k = threadIdx.x; k < half; k += kWavThreads) {
-      const int p = __ldg(kpos + k);
-      const int q = __ldg(kpos + (k ? N - k : 0));
-      const C fa = spectrum_at<R>(spa, k, N, adjoint);
-      const C zp = b[p];
-      const C zq = b[q];
-      if (wa == wb) {
-        b[p] = cmul(zp, fa);
-        if (q != p) b[q] = cmul(zq, cmake<C>(fa.x, -fa.y));
-      } else {
-        const C fb = spectrum_at<R>(spb, k, N, adjoint);
-        const C u = cmake<C>(zp.x + zq.x, zp.y - zq.y);  // Z_k + conj Z_{C-k}
-        const C d = cmake<C>(zp.x - zq.x, zp.y + zq.y);  // Z_k - conj Z_{C-k}
+  if (shared) {
+    pfa_turn_any<R, FMAX>(sh.f[0], buf, np, N, sh.g[0], sh.inv_lines[0], adjoint,
+                          [&](int pr) { return spectra + at[pr][0]; });
+    __syncthreads();
+  } else {
+    pfa_pass_any<R, false, FMAX>(sh.f[0], buf, np, N, sh.g[0], sh.inv_g[0], sh.inv_lines[0]);
+    __syncthreads();
+    // spectrum product (frequencies k and N - k together)
+    for (int pr = 0; pr < np; ++pr) {
+      const C *spa = spectra + at[pr][0];
+      const C *spb = spectra + at[pr][1];
+      C *b = buf + pr * N;
+      for (int k = threadIdx.x; k < N / 2 + 1; k += kWavThreads) {
+        const int p = __ldg(kpos + k);
+        const int q = __ldg(kpos + (k ? N - k : 0));
+        C fa = spa[p], fb = spb[p];
+        if (adjoint) {
+          fa.y = -fa.y;
+          fb.y = -fb.y;
+        }
+        const C zp = b[p];
+        const C zq = b[q];
+        const C u = cmake<C>(zp.x + zq.x, zp.y - zq.y);  // Z_k + conj Z_{N-k}
+        const C d = cmake<C>(zp.x - zq.x, zp.y + zq.y);  // Z_k - conj Z_{N-k}
         const C ua = cmul(u, fa);
         const C db = cmul(d, fb);
         b[p] = cmake<C>((R)0.5 * (ua.x + db.x), (R)0.5 * (ua.y + db.y));
-        // Z'_{C-k} = conj((u S_a - d S_b) / 2)
+        // Z'_{N-k} = conj((u S_a - d S_b) / 2)
         if (q != p) b[q] = cmake<C>((R)0.5 * (ua.x - db.x), (R)-0.5 * (ua.y - db.y));
       }
     }
+    __syncthreads();
+    pfa_pass_any<R, true, FMAX>(sh.f[0], buf, np, N, sh.g[0], sh.inv_g[0], sh.inv_lines[0]);
+    __syncthreads();
   }
-  __syncthreads();
-
-  for (int i = 0; i < sh.nf; ++i) {
+  for (int i = 1; i < sh.nf; ++i) {
     pfa_pass_any<R, true, FMAX>(sh.f[i], buf, np, N, sh.g[i], sh.inv_g[i], sh.inv_lines[i]);
     __syncthreads();
   }
@@ -263,26 +337,39 @@ __global__ void __launch_bounds__(kWavThreads, MINB)
   [[maybe_unused]] const int wrap = adjoint ? N - Ct : Ct;
   [[maybe_unused]] const int w_lo = adjoint ? 1 : 0;  // samples [w_lo, w_hi) take one
   [[maybe_unused]] const int w_hi = adjoint ? Ct : Ct - 1;
-  for (int pr = 0; pr < np; ++pr) {
-    const int ta = 2 * (pair0 + pr);
-    const bool has_b = ta + 1 < n_tr;
-    R *ya = job.y + (long)ta * Ct;
-    const C *b = buf + pr * N;
-    const bool live_a = job.src[ta] >= 0;
-    const bool live_b = has_b && job.src[ta + 1] >= 0;
-    for (int t = threadIdx.x; t < Ct; t += kWavThreads) {
-      C v = b[__ldg(qmap + t)];
-      if constexpr (PADDED) {
-        if (N != Ct && t >= w_lo && t < w_hi) v = cadd(v, b[__ldg(qmap + t + wrap)]);
+  {
+    bool live[kWavMaxPairs][2];
+#pragma unroll
+    for (int pr = 0; pr < kWavMaxPairs; ++pr)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int tr = 2 * (pair0 + pr) + h;
+        live[pr][h] = pr < np && tr < n_tr && job.src[tr] >= 0;
       }
-      if (live_a) ya[t] = v.x;
-      if (live_b) ya[Ct + t] = v.y;
+    R *y0 = job.y + 2L * pair0 * Ct;
+    for (int t = threadIdx.x; t < Ct; t += kWavThreads) {
+      const C *b = buf + __ldg(qmap + t);
+      const C *u = nullptr;
+      if constexpr (PADDED) {
+        if (N != Ct && t >= w_lo && t < w_hi) u = buf + __ldg(qmap + t + wrap);
+      }
+#pragma unroll
+      for (int pr = 0; pr < kWavMaxPairs; ++pr)
+        if (pr < np) {
+          C v = b[pr * N];
+          if constexpr (PADDED) {
+            if (u != nullptr) v = cadd(v, u[pr * N]);
+          }
+          R *y = y0 + 2L * pr * Ct + t;
+          if (live[pr][0]) y[0] = v.x;
+          if (live[pr][1]) y[Ct] = v.y;
+        }
     }
-    for (int h = 0; h < 2; ++h) {  // halves without a spectrum
-      if (h == 0 ? live_a : (live_b || !has_b)) continue;
-      for (int t = threadIdx.x; t < Ct; t += kWavThreads)
-        ya[h * Ct + t] = wavelet_input<R>(job, record, ta + h, t) * (R)Ct;
-    }
+  }
+  for (int tr = 2 * pair0; tr < min(2 * (pair0 + np), n_tr); ++tr) {  // without a spectrum
+    if (job.src[tr] >= 0) continue;
+    for (int t = threadIdx.x; t < Ct; t += kWavThreads)
+      job.y[(long)tr * Ct + t] = wavelet_input<R>(job, record, tr, t) * (R)Ct;
   }
 }
 
@@ -309,11 +396,13 @@ __global__ void __launch_bounds__(kWavThreads)
   if (threadIdx.x == 0) g[n] = t;
 }
 
-// Half spectrum of the taps zero-padded to length N, scaled by 1/N:
-// out[k] = (1/N) sum_{n<C} g[n] e^{-2 pi i n k / N}.  One block per bin.
+// Spectrum of the taps zero-padded to length N, scaled by 1/N, in the dense
+// frequency order: out[kpos[k]] = (1/N) sum_{n<C} g[n] e^{-2 pi i n k / N},
+// and its conjugate at kpos[N - k].  One block per k <= N / 2.
 template <typename R>
 __global__ void __launch_bounds__(kWavThreads)
-    wavelet_pad_spectrum(const double *__restrict__ g, int C, int N, Cx<R> *__restrict__ out) {
+    wavelet_pad_spectrum(const double *__restrict__ g, int C, int N,
+                         const unsigned short *__restrict__ kpos, Cx<R> *__restrict__ out) {
   __shared__ double red_c[32], red_s[32];
   const long k = blockIdx.x;
   double re = 0.0, im = 0.0;
@@ -325,7 +414,10 @@ __global__ void __launch_bounds__(kWavThreads)
   }
   const double tr = block_sum(re, red_c);
   const double ti = block_sum(im, red_s);
-  if (threadIdx.x == 0) out[k] = cmake<Cx<R>>((R)(tr / N), (R)(ti / N));
+  if (threadIdx.x == 0) {
+    out[kpos[k]] = cmake<Cx<R>>((R)(tr / N), (R)(ti / N));
+    if (k > 0 && 2 * k != N) out[kpos[N - k]] = cmake<Cx<R>>((R)(tr / N), (R)(-ti / N));
+  }
 }
 
 }  // namespace agd
