@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kPairThreads, MINB)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CxPair<R> *bins = reinterpret_cast<CxPair<R> *>(smem_raw);  // [f][pair]
   C *work = reinterpret_cast<C *>(bins + F * kPairs);
-  C *tw = work + S::kWork;  // W_N^k
+  C *tw = work + S::kWork;  // W_N^(m k) at 20 m + k
   __shared__ R taper[16 * NA];
   const TimeJob<R> &job = jobs[cta_job[blockIdx.x]];
   const int t0 = cta_trace0[blockIdx.x];
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kPairThreads, MINB)
   pair_range(job.T, t_begin, t_end);
   if (t_begin == t_end) return;
   for (int k = threadIdx.x; k < N; k += kPairThreads) {
-    tw[k] = ctw<R>(tw_offset(N) + k);
+    tw[k] = ctw<R>(tw_offset(N) + (k / 20) * (k % 20));
     if (k < 16 * NA) taper[k] = job.time_taper[k];
   }
   // copies in: pair cp, bins cf, cf + 20, ...
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kPairThreads, MINB)
       for (int m = 0; m < NA; ++m) {
         C u = v[m];
         if (m > 0) {
-          const C f = tw[m * cf];  // m cf < N
+          const C f = tw[20 * m + cf];
           u = cmake<C>(u.x * f.x + u.y * f.y, u.y * f.x - u.x * f.y);  // times conj W
         }
         w[m * kPairStride] = u;
@@ -195,7 +195,8 @@ __global__ void __launch_bounds__(kPairThreads, MINB)
   using S = TimePair<R, NA>;
   constexpr int N = S::N, F = S::F, H = S::H;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C *tw = reinterpret_cast<C *>(smem_raw);  // W_N^k
+  C *tw = reinterpret_cast<C *>(smem_raw);  // W_N^(m k) at NA m + k: neighbouring threads
+                                            // read neighbouring values
   C *work2 = tw + N;                        // two work buffers
   __shared__ R taper[16 * NA];
   const TimeJob<R> &job = jobs[cta_job[blockIdx.x]];
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(kPairThreads, MINB)
   pair_range(job.T, t_begin, t_end);
   if (t_begin == t_end) return;
   for (int k = threadIdx.x; k < N; k += kPairThreads) {
-    tw[k] = ctw<R>(tw_offset(N) + k);
+    tw[k] = ctw<R>(tw_offset(N) + (k / NA) * (k % NA));
     if (k < 16 * NA) taper[k] = job.time_taper[k];
   }
   // first pass: samples n2 + NA n1 of pair p, for NA * kPairs threads
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(kPairThreads, MINB)
       dft<R, 20, false>(v);
       C *w = work + n2 * kPairStride + p;
 #pragma unroll
-      for (int m = 0; m < 20; ++m) w[m * kPairs] = m > 0 ? cmul(v[m], tw[m * n2]) : v[m];
+      for (int m = 0; m < 20; ++m) w[m * kPairs] = m > 0 ? cmul(v[m], tw[NA * m + n2]) : v[m];
     }
     __syncthreads();
     C v[NA];
