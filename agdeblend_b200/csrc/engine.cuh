@@ -778,7 +778,8 @@ class Engine {
         add_adj_rows<2, 20, 40, 1, 256, 6, 2, 2>(c);
         add_adj_pipe<2, 20, 40, 1, 256, 6, 2>(c);
         add_adj_pipe<2, 20, 40, 1, 256, 5, 2, true>(c);
-        add_adj_pipe<2, 20, 40, 1, 256, 8, 2>(c);
+        add_adj_pipe<2, 20, 40, 1, 128, 4, 4>(c);
+        add_adj_pipe<2, 20, 40, 1, 64, 2, 8>(c);
       } else if (shape_is<2, 20, 20, 1>(W)) {
         add_fwd<2, 20, 20, 1, 384, 24, 2, 1>(c);
         add_fwd<2, 20, 20, 1, 256, 12, 1, 3>(c);
@@ -814,6 +815,7 @@ class Engine {
         add_adj_pipe<3, 20, 20, 20, 384, 1, 2>(c);
         add_adj_pipe<3, 20, 20, 20, 448, 1, 1, true>(c);
         add_adj_pipe<3, 20, 20, 20, 416, 1, 2>(c);
+        add_adj_pipe<3, 20, 20, 20, 320, 1, 2>(c);
       }
     } else {
       // double: the two-stage kernels only (one-stage kernels with several
