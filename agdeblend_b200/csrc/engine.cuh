@@ -561,7 +561,7 @@ class Engine {
     if (force != nullptr && force[0] != '\0') {
       pick = std::max(0, std::min(std::atoi(force), (int)cands.size() - 1));
     } else if (cands.size() > 1) {
-      pick = autotune_wavelet(cands.size(), n_max, [&](size_t v, TimeLaunch &L) {
+      pick = autotune_wavelet(cands.size(), fmax <= 17 ? 0 : 1, n_max, [&](size_t v, TimeLaunch &L) {
         launch_for(L, cands[v].np);
         return cands[v].fn;
       });
@@ -578,14 +578,14 @@ class Engine {
   // Times the wavelet candidates (both directions, three rounds, CUDA
   // events), cached per device, precision, trace length and size class.
   template <typename Make>
-  int autotune_wavelet(size_t n, int n_max, Make make) {
+  int autotune_wavelet(size_t n, int list, int n_max, Make make) {
     long traces = 0;
     for (const WindowPlan &W : plan.windows) traces += W.n_traces;
     int dev = 0;
     CK(cudaGetDevice(&dev));
     char key[96];
-    std::snprintf(key, sizeof key, "wav%d:%d:%d:%d:%d", wav_padded ? 1 : 0, dev, (int)sizeof(R), n_max,
-                  (int)std::log2((double)std::max(1L, traces)));
+    std::snprintf(key, sizeof key, "wav:%d:%d:%d:%d:%d:%d", dev, (int)sizeof(R), wav_padded ? 1 : 0,
+                  list, n_max, (int)std::log2((double)std::max(1L, traces)));
     static std::mutex mu;
     static std::map<std::string, int> cache;
     {
