@@ -1899,6 +1899,30 @@ class Engine {
 
   // ---------------------------------------------------------------- launches
 
+  // Launch of the kernels that begin with pdl_enter.  On small problems (model
+  // up to kPdlModelBytes) with programmatic stream serialization: the launch
+  // and the first instructions of a kernel overlap the end of the one before
+  // it, in a captured graph too (iteration of a 40-trace gather 20.5 -> 16.5
+  // us, of a 128-trace gather 26.7 -> 22.6, of a double one with a 9 MB model
+  // 91 -> 84).  On larger ones the waiting blocks take shared memory and L1
+  // from the running kernel: neutral from 20 MB (47 -> 48-51 us, 43 -> 41 us
+  // at 2.5 M complex) and slower beyond (two-volume survey 1050 -> 1210 us).
+  static constexpr size_t kPdlModelBytes = 16u << 20;
+  template <typename... P, typename... A>
+  void launch_pdl(void (*kernel)(P...), dim3 grid, int block, size_t smem, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = (size_t)plan.model_size * sizeof(C) <= kPdlModelBytes ? 1 : 0;
+    CK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+  }
+
   void launch_axis(const AxisLaunch &L, int inverse, int epilogue, R step, R lamb,
                    const R *lamb_dev = nullptr) {
     if (L.n_cta == 0) return;
@@ -1918,12 +1942,15 @@ class Engine {
   }
 
   // record <- sum of the window traces (muted with use_mute), minus d
-  void launch_record_gather(R *out, bool use_mute, const R *d, double *sumsq) {
-    if (g_fwd.n_chunk == 0) return;
-    record_gather<R><<<g_fwd.n_chunk, kThreads, 0, stream>>>(
-        g_fwd.runs.get(), g_fwd.chunk_ptr.get(), plan.record_size, Y.get(), out,
-        use_mute ? mute.get() : nullptr, d, sumsq);
-    CK(cudaGetLastError());
+  void launch_record_gather(R *out, bool use_mute, const R *d, double *sumsq,
+                            NextLambda<R> lambda = NextLambda<R>{}) {
+    if (g_fwd.n_chunk == 0) {
+      if (lambda.counter != nullptr) launch_pdl(next_lambda<R>, 1, 256, 0, lambda);
+      return;
+    }
+    launch_pdl(record_gather<R>, g_fwd.n_chunk, kThreads, 0, g_fwd.runs.get(),
+               g_fwd.chunk_ptr.get(), plan.record_size, Y.get(), out,
+               use_mute ? mute.get() : nullptr, d, sumsq, lambda);
   }
 
   void launch_space_fwd(const FastClass &c) {
@@ -1937,8 +1964,7 @@ class Engine {
       }
     }
     if (c.pl_fwd.n_batch == 0) return;
-    c.fv().fn<<<c.pl_fwd.grid, c.pl_fwd.nt, c.pl_fwd.smem, stream>>>(c.pl_fwd.batches());
-    CK(cudaGetLastError());
+    launch_pdl(c.fv().fn, c.pl_fwd.grid, c.pl_fwd.nt, c.pl_fwd.smem, c.pl_fwd.batches());
   }
 
   void launch_space_adj(const FastClass &c, const PlaneLaunch &L, int epilogue, R step, R lamb,
@@ -1955,10 +1981,8 @@ class Engine {
       }
     }
     if (L.n_batch == 0) return;
-    c.av().fn<<<L.grid, L.nt, L.smem, stream>>>(L.batches(), epilogue, step, lamb,
-                                                 multi ? step_dev.get() : nullptr, lamb_dev,
-                                                 multi ? pmax.get() : scalar.get());
-    CK(cudaGetLastError());
+    launch_pdl(c.av().fn, L.grid, L.nt, L.smem, L.batches(), epilogue, step, lamb,
+               multi ? step_dev.get() : nullptr, lamb_dev, multi ? pmax.get() : scalar.get());
   }
 
   // time c2r + taper + overlap-add of every window (fast time groups, then
@@ -1967,9 +1991,8 @@ class Engine {
     for (const auto &gp : tgroups) {
       const TimeGroup &g = *gp;
       if (!g.tf.n_cta) continue;
-      g.fwd<<<dim3(g.tf.n_cta, g.tf.splits), kPairThreads, g.tf.smem, stream>>>(
-          time_jobs.get(), g.tf.cta_job.get(), g.tf.cta_trace0.get());
-      CK(cudaGetLastError());
+      launch_pdl(g.fwd, dim3(g.tf.n_cta, g.tf.splits), kPairThreads, g.tf.smem, time_jobs.get(),
+                 g.tf.cta_job.get(), g.tf.cta_trace0.get());
     }
     if (time_fwd.n_cta) {
       time_c2r_ola<R><<<time_fwd.n_cta, kThreads, time_fwd.smem, stream>>>(
@@ -1985,9 +2008,8 @@ class Engine {
     for (const auto &gp : tgroups) {
       const TimeGroup &g = *gp;
       if (!g.ta.n_cta) continue;
-      g.adj<<<dim3(g.ta.n_cta, g.ta.splits), kPairThreads, g.ta.smem, stream>>>(
-          time_jobs.get(), g.ta.cta_job.get(), g.ta.cta_trace0.get(), record, from_record);
-      CK(cudaGetLastError());
+      launch_pdl(g.adj, dim3(g.ta.n_cta, g.ta.splits), kPairThreads, g.ta.smem, time_jobs.get(),
+                 g.ta.cta_job.get(), g.ta.cta_trace0.get(), record, from_record);
     }
     if (time_adj.n_cta) {
       time_r2c<R><<<time_adj.n_cta, kThreads, time_adj.smem, stream>>>(
@@ -2000,18 +2022,16 @@ class Engine {
   void launch_axis_dft(const AxisDftLaunch &L, bool forward) {
     if (L.b.n == 0) return;
     auto fn = forward ? axis_dft<R, true> : axis_dft<R, false>;
-    fn<<<L.b.grid, kDftThreads, L.b.smem, stream>>>(L.jobs.get(), L.b.job.get(), L.b.first.get(),
-                                                    L.b.n);
-    CK(cudaGetLastError());
+    launch_pdl(fn, L.b.grid, kDftThreads, L.b.smem, L.jobs.get(), L.b.job.get(),
+               L.b.first.get(), L.b.n);
   }
 
   void launch_plane_dft(const PlaneDftLaunch &L, bool line, bool forward, int epilogue, R step,
                         R lamb, const R *lamb_dev) {
     if (L.b.n == 0) return;
-    plane_kernel(line, forward)<<<L.b.grid, line ? line_nt : kDftThreads, L.b.smem, stream>>>(
-        L.jobs.get(), L.b.job.get(), L.b.first.get(), L.b.n, epilogue, step, lamb,
-        multi ? step_dev.get() : nullptr, lamb_dev, multi ? pmax.get() : scalar.get());
-    CK(cudaGetLastError());
+    launch_pdl(plane_kernel(line, forward), L.b.grid, line ? line_nt : kDftThreads, L.b.smem,
+               L.jobs.get(), L.b.job.get(), L.b.first.get(), L.b.n, epilogue, step, lamb,
+               multi ? step_dev.get() : nullptr, lamb_dev, multi ? pmax.get() : scalar.get());
   }
 
   void launch_dft_fwd() {
@@ -2051,10 +2071,8 @@ class Engine {
   // the window traces (direction -1, prime-factor kernel only)
   void launch_wavelet_fast(int direction, const R *record) {
     if (!wavf.n_cta) return;
-    wav_fn<<<wavf.n_cta, kWavThreads, wavf.smem, stream>>>(
-        wavf_jobs.get(), wavf.cta_job.get(), wavf.cta_trace0.get(), wavf.nb, spectra.get(),
-        spec_off.get(), direction, record);
-    CK(cudaGetLastError());
+    launch_pdl(wav_fn, wavf.n_cta, kWavThreads, wavf.smem, wavf_jobs.get(), wavf.cta_job.get(),
+               wavf.cta_trace0.get(), wavf.nb, spectra.get(), spec_off.get(), direction, record);
   }
 
   void launch_wavelet(int direction) {
@@ -2101,15 +2119,15 @@ class Engine {
     for (int k = 0; k < 2; ++k) n += (dft_fwd[k].b.n ? 1 : 0) + (dft_adj[k].b.n ? 1 : 0);
     n += (int)(dft_fwd_axes.size() + dft_adj_axes.size());
     n += (time_fwd.n_cta ? 1 : 0) + (time_adj.n_cta ? 1 : 0);
-    n += (g_fwd.n_chunk ? 1 : 0) + 1;  // residual gather, threshold schedule
+    n += 1;  // residual gather with the threshold schedule
     if (wavelets) n += wav_fast ? 2 : 3;
     return n;
   }
 
   // ---------------------------------------------------------------- graphs
 
-  // One ISTA iteration (forward, residual, next lambda, adjoint update)
-  // captured once and replayed; lambda comes from a device table indexed by
+  // One ISTA iteration (forward, residual with the next lambda, adjoint
+  // update) captured once and replayed; lambda comes from a device table indexed by
   // a device counter the graph advances.
   DevArray<R> lamb_table, lamb_cur;
   DevArray<int> lamb_counter;
@@ -2141,10 +2159,7 @@ class Engine {
 
   void iteration_body(bool want_norm) {
     forward_traces();
-    residual(want_norm);
-    next_lambda<R><<<1, 256, 0, stream>>>(lamb_table.get(), lamb_counter.get(), lamb_cur.get(),
-                                          plan.n_problems);
-    CK(cudaGetLastError());
+    residual(want_norm, true);
     adjoint_update(rec_r.get(), stepsize, (R)0, false, lamb_cur.get());
   }
 
@@ -2167,13 +2182,34 @@ class Engine {
 
   void replay_iteration() { CK(cudaGraphLaunch(iter_graph, stream)); }
 
-  void residual(bool want_norm) {
+  // n iterations, as replays of the captured graph.  A short solve without a
+  // graph launches its kernels directly: the capture costs about 120 us, a
+  // replay saves about 2.5 us of launch time (29 iterations of a 40-trace
+  // gather: 1.33 ms per call captured, 1.21 direct; 99 of a 128-trace gather:
+  // 3.06 and 3.19).
+  static constexpr int kGraphIterations = 48;
+  void run_iterations(int n) {
+    if (n < kGraphIterations && iter_graph == nullptr) {
+      for (int i = 0; i < n; ++i) iteration_body(false);
+      return;
+    }
+    capture_iteration();
+    for (int i = 0; i < n; ++i) replay_iteration();
+  }
+
+  // r = A x - d (want_norm: its squared norm in dscalar); advance: also the
+  // next threshold of the schedule
+  void residual(bool want_norm, bool advance = false) {
     double *ss = nullptr;
     if (want_norm) {
       CK(cudaMemsetAsync(dscalar.get(), 0, sizeof(double), stream));
       ss = dscalar.get();
     }
-    launch_record_gather(rec_r.get(), true, rec_d.get(), ss);
+    NextLambda<R> lambda{};
+    if (advance)
+      lambda = NextLambda<R>{lamb_table.get(), lamb_counter.get(), lamb_cur.get(),
+                             plan.n_problems};
+    launch_record_gather(rec_r.get(), true, rec_d.get(), ss, lambda);
   }
 
   double read_dscalar() {
@@ -2419,9 +2455,8 @@ class Engine {
           std::printf("Iteration %d Residual %f\n", it, r);
         }
       }
-    } else if (end > first) {
-      capture_iteration();
-      for (int it = first; it < end; ++it) replay_iteration();
+    } else {
+      run_iterations(end - first);
     }
     if (model_out != nullptr) model_to_ref(X.get(), model_out);
     output();
@@ -2527,9 +2562,8 @@ class Engine {
           std::printf("Iteration %d Residual %f\n", it, r);
         }
       }
-    } else if (n_its > begin) {
-      capture_iteration();
-      for (int it = begin; it < n_its; ++it) replay_iteration();
+    } else {
+      run_iterations(n_its - begin);
     }
     output();
     check_tc_error();

@@ -529,6 +529,7 @@ __global__ void __launch_bounds__(NT, MINB) space_fwd_fast(PlaneBatches<R> batch
   constexpr int LL = PL * 4 / 5;         // cropped row
   constexpr int ORW = S::dense_L / LL;   // cropped rows per plane
   static_assert(LL % 2 == 0, "cropped rows of column pairs");
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *stage[2] = {reinterpret_cast<C *>(smem_raw),
                  reinterpret_cast<C *>(smem_raw) + (STAGES == 2 ? NP * S::size : 0)};
@@ -626,6 +627,7 @@ __global__ void __launch_bounds__(NT, MINB)
   static_assert(STAGES == 1 || STAGES == 2, "one or two stages");
   using C = Cx<R>;
   using S = PlaneShape<D, P0, P1, P2>;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *base = reinterpret_cast<C *>(smem_raw);
   C *stage[2] = {base, base + (STAGES == 2 ? NP * S::size : 0)};
@@ -782,6 +784,7 @@ __global__ void __launch_bounds__(NT, MINB) space_fwd_rows(PlaneBatches<R> batch
   constexpr int PL = S::PL;                      // last-axis padded length
   constexpr int LL = PL * 4 / 5;                 // its window length
   constexpr int ROWS = S::dense_P / PL;          // rows per model plane
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *buf = reinterpret_cast<C *>(smem_raw);
   for (int b = blockIdx.x; b < batches.n; b += gridDim.x) {
@@ -836,6 +839,7 @@ __global__ void __launch_bounds__(NT, MINB)
   constexpr int PL = S::PL;
   constexpr int LL = PL * 4 / 5;
   constexpr int ROWS = S::dense_P / PL;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *base = reinterpret_cast<C *>(smem_raw);
   C *stage[2] = {base, base + (STAGES == 2 ? NP * Z : 0)};
@@ -1012,6 +1016,7 @@ __global__ void __launch_bounds__(NT, MINB)
   constexpr bool kVec = sizeof(R) == sizeof(float) && PL % 2 == 0;
   constexpr int kStg = NP * S::dense_L + (NP * S::dense_L) % 2;  // 16-byte aligned
   constexpr int kWork = NP * Z + (NP * Z) % 2;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *stg = reinterpret_cast<C *>(smem_raw);
   C *work = stg + kStg;

@@ -23,6 +23,20 @@ namespace agd {
 
 constexpr int kThreads = 256;
 
+// ------------------------------------------------------------ launches
+
+// First statement of the kernels of an iteration, which are launched with
+// programmatic stream serialization: the next kernel may be launched from
+// here on (its blocks start as this one's make room and wait in their own
+// pdl_enter), and everything before this kernel is complete and visible
+// after it.  Every block passes it before it returns, so that a kernel's
+// completion implies its predecessors'.  Only tables that no kernel writes
+// may be read before it.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ------------------------------------------------------------ job records
 
 // One window's pass along one space axis.  Lines are indexed q = o*inner + i
@@ -550,6 +564,26 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// Advances the threshold schedule on the device: out[0..n) = row *counter of
+// table (n thresholds per iteration, one per problem solved together), then
+// ++*counter.  Carried out by one block of the iteration's residual gather,
+// between the adjoint of the last iteration and that of this one, which read
+// out.
+template <typename R>
+struct NextLambda {
+  const R *table;
+  int *counter;  // NULL: nothing to do
+  R *out;
+  int n;
+
+  __device__ __forceinline__ void advance() const {
+    const int k = *counter;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) out[i] = table[(long)k * n + i];
+    __syncthreads();
+    if (threadIdx.x == 0) *counter = k + 1;
+  }
+};
+
 // The forward operator's gather: record[s] = sum of the window traces'
 // samples at s, in list order (the serial reference's window-then-trace
 // order), minus d with the residual, zero where muted.  Block b owns the
@@ -572,8 +606,11 @@ template <typename R>
 __global__ void __launch_bounds__(kThreads)
     record_gather(const GatherRun *__restrict__ runs, const long *__restrict__ chunk_ptr,
                   long record_size, const R *__restrict__ src, R *__restrict__ out,
-                  const uint8_t *__restrict__ mute, const R *__restrict__ d, double *sumsq) {
+                  const uint8_t *__restrict__ mute, const R *__restrict__ d, double *sumsq,
+                  NextLambda<R> lambda) {
   __shared__ GatherRun tile[kGatherTile];
+  pdl_enter();
+  if (lambda.counter != nullptr && blockIdx.x == 0) lambda.advance();
   const long s0 = (long)blockIdx.x * kRecordChunk + threadIdx.x;
   const long b0 = chunk_ptr[blockIdx.x];
   const long b1 = chunk_ptr[blockIdx.x + 1];
@@ -693,15 +730,10 @@ __global__ void record_sumsq(const R *__restrict__ x, long n, double *out) {
   if (threadIdx.x == 0) atomicAdd(out, s);
 }
 
-// Advances the threshold schedule on the device: out[0..n) = row *counter
-// of table (n thresholds per iteration, one per problem solved together),
-// then ++*counter.  One block; captured in the per-iteration CUDA graph.
+// The schedule step alone, for problems without a record.
 template <typename R>
-__global__ void next_lambda(const R *__restrict__ table, int *counter, R *out, int n) {
-  const int k = *counter;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) out[i] = table[(long)k * n + i];
-  __syncthreads();
-  if (threadIdx.x == 0) *counter = k + 1;
+__global__ void next_lambda(NextLambda<R> lambda) {
+  lambda.advance();
 }
 
 // Window traces from patch data (the transpose of output_gather): for every

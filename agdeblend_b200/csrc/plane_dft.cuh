@@ -419,6 +419,7 @@ __global__ void __launch_bounds__(kDftThreads, sizeof(R) == sizeof(float) ? 4 : 
               const long *__restrict__ batch_plane, int n_batch, int epilogue, R step_arg,
               R lamb_arg, const R *step_dev, const R *lamb_dev, R *max_out) {
   using C = Cx<R>;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const bool multi = step_dev != nullptr;
   R *const smem = reinterpret_cast<R *>(smem_raw);
@@ -522,6 +523,7 @@ __global__ void __launch_bounds__(NT, (sizeof(R) == sizeof(float) ? 512 : 384) /
              const long *__restrict__ batch_line, int n_batch, int epilogue, R step_arg,
              R lamb_arg, const R *step_dev, const R *lamb_dev, R *max_out) {
   using C = Cx<R>;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const bool multi = step_dev != nullptr;
   R *const tab = reinterpret_cast<R *>(smem_raw);
@@ -573,6 +575,7 @@ __global__ void __launch_bounds__(kDftThreads, sizeof(R) == sizeof(float) ? 4 : 
     axis_dft(const AxisDftJob<R> *__restrict__ jobs, const int *__restrict__ batch_job,
              const long *__restrict__ batch_line, int n_batch) {
   using C = Cx<R>;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R *const smem = reinterpret_cast<R *>(smem_raw);
   auto fetch = [&](int bi, int half) {

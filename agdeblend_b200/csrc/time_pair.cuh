@@ -83,11 +83,12 @@ __global__ void __launch_bounds__(kPairThreads, MINB)
   const int nb = min(2 * kPairs, ntr - t0);
   int t_begin, t_end;
   pair_range(job.T, t_begin, t_end);
-  if (t_begin == t_end) return;
   for (int k = threadIdx.x; k < N; k += kPairThreads) {
     tw[k] = ctw<R>(tw_offset(N) + (k / 20) * (k % 20));
     if (k < 16 * NA) taper[k] = job.time_taper[k];
   }
+  pdl_enter();
+  if (t_begin == t_end) return;
   // copies in: pair cp, bins cf, cf + 20, ...
   const int cp = threadIdx.x % kPairs;
   const int cf = threadIdx.x / kPairs;
@@ -205,11 +206,12 @@ __global__ void __launch_bounds__(kPairThreads, MINB)
   const int nb = min(2 * kPairs, ntr - t0);
   int t_begin, t_end;
   pair_range(job.T, t_begin, t_end);
-  if (t_begin == t_end) return;
   for (int k = threadIdx.x; k < N; k += kPairThreads) {
     tw[k] = ctw<R>(tw_offset(N) + (k / NA) * (k % NA));
     if (k < 16 * NA) taper[k] = job.time_taper[k];
   }
+  pdl_enter();
+  if (t_begin == t_end) return;
   // first pass: samples n2 + NA n1 of pair p, for NA * kPairs threads
   const int n2 = threadIdx.x % NA;
   const int p = threadIdx.x / NA;

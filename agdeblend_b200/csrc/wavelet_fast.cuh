@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(kWavThreads, MINB)
                  const Cx<R> *__restrict__ spectra, const long *__restrict__ spec_off,
                  int direction, const R *__restrict__ record) {
   using C = Cx<R>;
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *buf = reinterpret_cast<C *>(smem_raw);
   const WaveletFastJob<R> &job = jobs[cta_job[blockIdx.x]];
