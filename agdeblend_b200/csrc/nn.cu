@@ -136,8 +136,8 @@ cudaError_t launch_gemm(const uint16_t *A, const uint16_t *B, float *C, int M, i
     agd::tc_gemm_bf16<BN><<<grid, 128, L::kBytes, s>>>(A, B, ws, M, N, K, lda, ldb, ldc, alpha,
                                                         0.f, k_split, slice, conv, act, err);
     const long total = (long)M * N;
-    const unsigned g = (unsigned)std::max<long>(1, std::min<long>((total + 255) / 256, 148L * 8));
-    agd::split_reduce<<<g, 256, 0, s>>>(ws, splits, slice, M, N, ldc, C, beta);
+    const unsigned g = (unsigned)std::max<long>(1, std::min<long>((total + 31) / 32, 148L * 8));
+    agd::split_reduce<<<g, 32 * agd::kReduceWays, 0, s>>>(ws, splits, slice, M, N, ldc, C, beta);
     return cudaGetLastError();
   }
   agd::tc_gemm_bf16<BN><<<grid, 128, L::kBytes, s>>>(A, B, C, M, N, K, lda, ldb, ldc, alpha,
@@ -701,19 +701,25 @@ class Net {
     act_backward<<<grid_of(P * L.cout_s), kNnThreads, 0, s>>>(Y.g.get(), Y.v.get(), P, L.cout,
                                                                L.cout_s, L.relu, dz.get());
     NCK(cudaGetLastError());
-    bias_grad<<<L.cout, kNnThreads, 0, s>>>(dz.get(), P, L.cout, L.cout_s,
-                                            grad.get() + L.b_off);
-    NCK(cudaGetLastError());
-    // dW = dZ^T col: both transposed so that the pixels are the K dimension
-    im2col3x3<<<grid_of(P * L.kp), kNnThreads, 0, s>>>(X.v.get(), cur_n, H, Wd, L.cin, X.Cs,
-                                                       L.kp, col.get());
-    NCK(cudaGetLastError());
+    // dW = dZ^T col with the pixels as the K dimension: dZ transposed, and
+    // the transposed im2col matrix from the transposed activations (in `col`,
+    // which the backward pass does not use otherwise)
     const dim3 tb(32, 8);
-    transpose_bf16<<<dim3((unsigned)((P + 31) / 32), (unsigned)((L.kp + 31) / 32)), tb, 0, s>>>(
-        col.get(), P, L.kp, L.kp, colT.get(), P);
-    NCK(cudaGetLastError());
     transpose_bf16<<<dim3((unsigned)((P + 31) / 32), (unsigned)((L.cout_s + 31) / 32)), tb, 0,
                      s>>>(dz.get(), P, L.cout_s, L.cout_s, dzT.get(), P);
+    NCK(cudaGetLastError());
+    const int chunks = (int)((P + kBiasChunk - 1) / kBiasChunk);
+    bias_partial<<<dim3((unsigned)chunks, (unsigned)L.cout), kNnThreads, 0, s>>>(dzT.get(), P,
+                                                                               dcol.get());
+    NCK(cudaGetLastError());
+    bias_sum<<<(L.cout + 31) / 32, 32, 0, s>>>(dcol.get(), chunks, L.cout, grad.get() + L.b_off);
+    NCK(cudaGetLastError());
+    transpose_bf16<<<dim3((unsigned)((P + 31) / 32), (unsigned)((L.cin + 31) / 32)), tb, 0, s>>>(
+        X.v.get(), P, L.cin, X.Cs, col.get(), P);
+    NCK(cudaGetLastError());
+    const long groups = ((P + 7) / 8 + kNnThreads - 1) / kNnThreads;
+    im2col3x3_t<<<dim3((unsigned)std::min<long>(groups, 148L * 8), (unsigned)L.kp), kNnThreads, 0,
+                  s>>>(col.get(), cur_n, H, Wd, L.cin, L.kp, colT.get());
     NCK(cudaGetLastError());
     NCK(cudaMemsetAsync(dwp.get(), 0, (size_t)L.cout_s * L.kp * sizeof(float), s));
     const long tiles = ((L.cout_s + 127) / 128) * ((L.kp + (L.kp <= 64 ? 63 : 127)) /
@@ -727,8 +733,12 @@ class Net {
     if (!need_dx) return;
     // dX = col2im(dZ W)
     gemm(dz.get(), wpt[li].get(), dcol.get(), P, L.kp, L.cout_s, L.cout_s, L.cout_s, L.kp, 0.f);
-    col2im3x3<<<grid_of(P * L.cin), kNnThreads, 0, s>>>(dcol.get(), cur_n, H, Wd, L.cin, L.kp,
-                                                        t[L.in].g.get(), X.Cs, 1);
+    if (L.cin % 4 == 0 && X.Cs % 4 == 0 && L.kp % 4 == 0)
+      col2im3x3_v4<<<grid_of(P * (L.cin / 4)), kNnThreads, 0, s>>>(
+          dcol.get(), cur_n, H, Wd, L.cin, L.kp, t[L.in].g.get(), X.Cs);
+    else
+      col2im3x3<<<grid_of(P * L.cin), kNnThreads, 0, s>>>(
+          dcol.get(), cur_n, H, Wd, L.cin, L.kp, t[L.in].g.get(), X.Cs, 1);
     NCK(cudaGetLastError());
   }
 
