@@ -224,10 +224,20 @@ class Engine {
   // own static shared memory; smem_max becomes the smallest such limit.
   template <typename K>
   int opt_in(K kernel, int limit) {
+    // once per kernel and device: the attribute stays
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, int> done;
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    const std::pair<int, const void *> key(dev, reinterpret_cast<const void *>(kernel));
+    std::lock_guard<std::mutex> lk(mu);
+    const auto it = done.find(key);
+    if (it != done.end()) return it->second;
     cudaFuncAttributes fa;
     CK(cudaFuncGetAttributes(&fa, kernel));
     const int dyn = limit - (int)fa.sharedSizeBytes;
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+    done[key] = dyn;
     return dyn;
   }
 
@@ -262,6 +272,12 @@ class Engine {
   // twiddle tables of the register DFTs in constant memory of the current
   // device (fast.cuh), shared by the fast space, time and wavelet kernels
   void upload_twiddles() {
+    static std::mutex mu;
+    static std::map<int, bool> done;  // per device: the tables stay
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    if (done[dev]) return;
     std::vector<C> tw(kTwTotal);
     for (int i = 0, off = 0; i < kNumTw; off += kTwSizes[i], ++i)
       for (int k = 0; k < kTwSizes[i]; ++k) {
@@ -270,9 +286,13 @@ class Engine {
         tw[off + k].y = (R)std::sin(a);
       }
     if (sizeof(R) == sizeof(float))
-      CK(cudaMemcpyToSymbol(c_tw_f, tw.data(), tw.size() * sizeof(C)));
+      CK(cudaMemcpyToSymbolAsync(c_tw_f, tw.data(), tw.size() * sizeof(C), 0,
+                                 cudaMemcpyHostToDevice, stream));
     else
-      CK(cudaMemcpyToSymbol(c_tw_d, tw.data(), tw.size() * sizeof(C)));
+      CK(cudaMemcpyToSymbolAsync(c_tw_d, tw.data(), tw.size() * sizeof(C), 0,
+                                 cudaMemcpyHostToDevice, stream));
+    CK(cudaStreamSynchronize(stream));
+    done[dev] = true;
   }
 
   // C = product of pairwise coprime prime powers with a register DFT; the
@@ -1662,14 +1682,14 @@ class Engine {
 
     setup_mark("tables");
     pick_classes();
-    X.alloc_pooled(M);
-    S0.alloc_pooled(M);
+    X.alloc(M);
+    S0.alloc(M);
     bool second = n_generic > 0;  // a second intermediate: generic passes, single-axis passes
     for (int w = 0; w < nw; ++w) second = second || (win_dft[w] && plan.windows[w].D > win_dft[w]);
-    if (second) S1.alloc_pooled(M);
-    Y.alloc_pooled(toff);
-    rec_d.alloc_pooled(plan.record_size);
-    rec_r.alloc_pooled(plan.record_size);
+    if (second) S1.alloc(M);
+    Y.alloc(toff);
+    rec_d.alloc(plan.record_size);
+    rec_r.alloc(plan.record_size);
     scalar.alloc(1);
     dscalar.alloc(1);
     multi = plan.n_problems > 1;
@@ -1818,7 +1838,7 @@ class Engine {
       poff += (long)plan.n_traces[p] * plan.n_times[p];
     }
     data_size = poff;
-    data_dev.alloc_pooled(data_size);
+    data_dev.alloc(data_size);
     {
       std::vector<std::vector<long>> cover;  // per global patch trace
       std::vector<long> tr_base(plan.n_patches);
@@ -1862,7 +1882,7 @@ class Engine {
 
   void ensure_plain_adjoint() {
     if (G.get() != nullptr || plan.model_size == 0) return;
-    G.alloc_pooled(plan.model_size);
+    G.alloc(plan.model_size);
     for (auto &cp : classes) {
       FastClass &c = *cp;
       std::vector<PlaneJob<R>> jobs = c.plain_jobs;

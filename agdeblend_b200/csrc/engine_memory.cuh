@@ -72,16 +72,20 @@ static void check(cudaError_t e, const char *what) {
 #define CK(x) check((x), #x)
 
 // Device blocks of finished problems kept for the next problem on the same
-// device: a deblending call allocates its large arrays (model, intermediates,
-// traces, records) once per call, and a fresh cudaMalloc of gigabytes costs
-// page mapping that can exceed the solve itself.  Blocks enter the cache
-// only from the destructor of an engine whose stream has been synchronised,
-// so no kernel can still use them.  Best fit within a factor of two; at most
+// device: a deblending call allocates its arrays once per call, a fresh
+// cudaMalloc of gigabytes costs page mapping that can exceed the solve
+// itself, and the fifty small tables of a 40-trace gather cost 0.3 ms of a
+// 1.1 ms call in cudaMalloc and cudaFree.  Blocks enter the cache only when
+// the work of their engine's stream that used them has been waited for, so
+// no kernel can still use them.  Sizes are rounded up to kGrain.  Best fit within a factor of two; at most
 // half the device memory is held (AGD_GPU_CACHE=0 disables the cache;
 // agd_gpu_release_cache frees it).
 class DevicePool {
  public:
+  static constexpr size_t kGrain = 512;
+
   static void *take(size_t bytes) {
+    bytes = (bytes + kGrain - 1) / kGrain * kGrain;
     if (injected_alloc_failure()) throw DeviceError("injected device allocation failure");
     int dev = 0;
     CK(cudaGetDevice(&dev));
@@ -214,39 +218,27 @@ class DevArray {
   DevArray() = default;
   DevArray(const DevArray &) = delete;
   DevArray &operator=(const DevArray &) = delete;
-  DevArray(DevArray &&o) noexcept : p_(o.p_), n_(o.n_), pooled_(o.pooled_) {
+  DevArray(DevArray &&o) noexcept : p_(o.p_), n_(o.n_) {
     o.p_ = nullptr;
     o.n_ = 0;
-    o.pooled_ = false;
   }
   DevArray &operator=(DevArray &&o) noexcept {
     if (this != &o) {
       release();
       p_ = o.p_;
       n_ = o.n_;
-      pooled_ = o.pooled_;
       o.p_ = nullptr;
       o.n_ = 0;
-      o.pooled_ = false;
     }
     return *this;
   }
   ~DevArray() { release(); }
+  // From the device cache; when the array is released, the work on its
+  // engine's stream that uses it must have been waited for (engine members:
+  // the engine synchronises before destruction).
   void alloc(size_t n) {
     release();
-    if (n && injected_alloc_failure())
-      throw DeviceError("injected device allocation failure");
-    if (n) CK(cudaMalloc(reinterpret_cast<void **>(&p_), n * sizeof(T)));
-    n_ = n;
-  }
-  // From the device cache; the array must live until its engine's stream
-  // is idle (engine members: the engine synchronises before destruction).
-  void alloc_pooled(size_t n) {
-    release();
-    if (n) {
-      p_ = static_cast<T *>(DevicePool::take(n * sizeof(T)));
-      pooled_ = true;
-    }
+    if (n) p_ = static_cast<T *>(DevicePool::take(n * sizeof(T)));
     n_ = n;
   }
   void upload(const std::vector<T> &v, cudaStream_t s) {
@@ -257,21 +249,14 @@ class DevArray {
   size_t size() const { return n_; }
   size_t bytes() const { return n_ * sizeof(T); }
   void release() {
-    if (p_) {
-      if (pooled_)
-        DevicePool::put(p_);
-      else
-        cudaFree(p_);
-    }
+    if (p_) DevicePool::put(p_);
     p_ = nullptr;
     n_ = 0;
-    pooled_ = false;
   }
 
  private:
   T *p_ = nullptr;
   size_t n_ = 0;
-  bool pooled_ = false;
 };
 
 // Distinct FFT lengths with their radix lists and twiddle tables.
