@@ -1069,10 +1069,13 @@ class Engine {
       }
     pick_plane_batches(jf[0]);
     pick_plane_batches(ja[0]);
-    // lines: 256-thread blocks share the tables of long axes
+    // lines: 256-thread blocks share the tables of long axes in float; the
+    // doubles' registers leave 384 threads per SM, three blocks of 128 (a
+    // 217-trace gather: 405 batches in one round of 444 blocks, 24 and 25 us;
+    // in three rounds of 148 blocks of 256 threads 33 and 38 us)
     int table = 0;
     for (const auto &j : jf[1]) table = std::max(table, dft_table_reals(j.b));
-    line_nt = table * sizeof(R) > 8192 ? 256 : 128;
+    line_nt = sizeof(R) == sizeof(float) && table * sizeof(R) > 8192 ? 256 : 128;
     pick_line_batches(jf[1]);
     pick_line_batches(ja[1]);
     for (int k = 0; k < 2; ++k) {
@@ -1147,7 +1150,8 @@ class Engine {
   void pick_line_batches(std::vector<PlaneDftJob<R>> &jobs) const {
     long total = 0;
     for (const auto &j : jobs) total += j.planes;
-    const long cap = std::max<long>(4, total / (512 / line_nt * (long)n_sm) / 4 * 4);
+    const long resident = (sizeof(R) == sizeof(float) ? 512 : 384) / line_nt * (long)n_sm;
+    const long cap = std::max<long>(4, (total / resident + 4) / 4 * 4);
     for (auto &j : jobs) {
       long nl = std::min<long>(4L * (line_nt / (j.b.kpad / kDftTk<R>)), cap);
       while (nl > 4 && line_dft_smem<R>(j.b, nl) > dft_budget(line_nt)) nl -= 4;
