@@ -838,20 +838,29 @@ class Engine {
         add_adj_pipe<3, 20, 20, 20, 320, 1, 2>(c);
       }
     } else {
-      // double: the two-stage kernels only (one-stage kernels with several
-      // blocks per SM would spill), and one stage for the 20x20x20 planes
+      // double: two stages with one block per SM, and one-stage and pipelined
+      // kernels in blocks small enough for 255 registers per thread
       if (shape_is<1, 40, 1, 1>(W)) {
         add_fwd<1, 40, 1, 1, 256, 128, 2, 1>(c);
         add_adj<1, 40, 1, 1, 192, 96, 2, 1>(c);
+        add_fwd<1, 40, 1, 1, 64, 64, 1, 4>(c);
+        add_adj_pipe<1, 40, 1, 1, 64, 32, 4>(c);
       } else if (shape_is<1, 20, 1, 1>(W)) {
         add_fwd<1, 20, 1, 1, 256, 256, 2, 1>(c);
         add_adj<1, 20, 1, 1, 256, 160, 2, 1>(c);
       } else if (shape_is<2, 20, 40, 1>(W)) {
         add_fwd<2, 20, 40, 1, 384, 8, 2, 1>(c);
         add_adj<2, 20, 40, 1, 384, 5, 2, 1>(c);
+        add_fwd<2, 20, 40, 1, 128, 6, 1, 2>(c);
+        add_fwd<2, 20, 40, 1, 64, 3, 1, 4>(c);
+        add_adj_pipe<2, 20, 40, 1, 128, 4, 2>(c);
+        add_adj_pipe<2, 20, 40, 1, 64, 2, 4>(c);
+        add_adj_pipe<2, 20, 40, 1, 80, 2, 3>(c);
       } else if (shape_is<2, 20, 20, 1>(W)) {
         add_fwd<2, 20, 20, 1, 384, 12, 2, 1>(c);
         add_adj<2, 20, 20, 1, 384, 10, 2, 1>(c);
+        add_fwd<2, 20, 20, 1, 128, 6, 1, 4>(c);
+        add_adj_pipe<2, 20, 20, 1, 128, 6, 3>(c);
       } else if (shape_is<2, 40, 40, 1>(W)) {
         add_fwd<2, 40, 40, 1, 320, 4, 2, 1>(c);
         add_adj<2, 40, 40, 1, 256, 2, 2, 1>(c);

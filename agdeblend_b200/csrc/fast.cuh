@@ -22,6 +22,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "kernels.cuh"
 
@@ -1006,14 +1007,17 @@ __global__ void __launch_bounds__(NT, MINB)
   constexpr int PLS = S::PLS;
   constexpr int ROWS = S::dense_P / PL;
   static_assert(Z == ROWS * PLS, "padded rows evenly spaced");
-  constexpr int CW = PL / 2;               // 16-byte columns of a row (float)
+  constexpr int EV = sizeof(C) == 8 ? 2 : 1;  // values of a 16-byte column
+  using Col = typename std::conditional<EV == 2, float4, C>::type;
+  constexpr int CW = PL / EV;              // 16-byte columns of a row
   constexpr int TR = NT / CW;              // rows per sweep
   // model loads in flight per thread (XS false), and whether the first ones
   // are issued before the last pass, from the register budget
   constexpr int kRegs = 65536 / (NT * MINB);
   constexpr int U = XS ? 1 : (kRegs >= 120 && PL <= 20 ? 8 : 4);
-  constexpr bool kEarly = !XS && D > 1 && 2 * PL + 4 * U + 24 <= kRegs;
-  constexpr bool kVec = sizeof(R) == sizeof(float) && PL % 2 == 0;
+  constexpr bool kEarly =
+      !XS && D > 1 && (int)(sizeof(C) / 4) * PL + 4 * U + 24 <= kRegs;
+  constexpr bool kVec = PL % EV == 0;
   constexpr int kStg = NP * S::dense_L + (NP * S::dense_L) % 2;  // 16-byte aligned
   constexpr int kWork = NP * Z + (NP * Z) % 2;
   pdl_enter();
@@ -1082,13 +1086,13 @@ __global__ void __launch_bounds__(NT, MINB)
     }
     const int nrows = np * ROWS;
     const bool vec = kVec && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
-    float4 xv[U];
+    Col xv[U];
     auto load_x = [&](int r0) {
 #pragma unroll
       for (int j = 0; j < U; ++j) {
         const int r = r0 + rr + TR * j;
         if (lane_on && r < nrows)
-          xv[j] = reinterpret_cast<const float4 *>(XS ? xbuf : dst)[r * CW + col];
+          xv[j] = reinterpret_cast<const Col *>(XS ? xbuf : dst)[r * CW + col];
       }
     };
     if (kEarly && vec && need_x) load_x(0);
@@ -1107,27 +1111,43 @@ __global__ void __launch_bounds__(NT, MINB)
         for (int j = 0; j < U; ++j) {
           const int r = r0 + rr + TR * j;
           if (!lane_on || r >= nrows) continue;
-          const C g0 = work[r * PLS + 2 * col];
-          const C g1 = work[r * PLS + 2 * col + 1];
-          float4 *d4 = reinterpret_cast<float4 *>(dst) + r * CW + col;
-          if (!need_x) {
-            *d4 = make_float4((float)g0.x, (float)g0.y, (float)g1.x, (float)g1.y);
-            continue;
-          }
-          C n0 = cmake<C>(sub_rn<R>((R)xv[j].x, mul_rn<R>(step, g0.x)),
-                          sub_rn<R>((R)xv[j].y, mul_rn<R>(step, g0.y)));
-          C n1 = cmake<C>(sub_rn<R>((R)xv[j].z, mul_rn<R>(step, g1.x)),
-                          sub_rn<R>((R)xv[j].w, mul_rn<R>(step, g1.y)));
-          if (epilogue == kUpdateThreshold) {
-            n0 = soft_threshold<R>(n0, lamb, lamb_sq);
-            n1 = soft_threshold<R>(n1, lamb, lamb_sq);
+          if constexpr (EV == 1) {
+            C *d = dst + r * CW + col;
+            C n = work[r * PLS + col];
+            if (need_x) {
+              n = cmake<C>(sub_rn<R>(xv[j].x, mul_rn<R>(step, n.x)),
+                           sub_rn<R>(xv[j].y, mul_rn<R>(step, n.y)));
+              if (epilogue == kUpdateThreshold) {
+                n = soft_threshold<R>(n, lamb, lamb_sq);
+              } else {
+                const R a2 = abs_sq<R>(n);
+                local_max = a2 > local_max ? a2 : local_max;
+              }
+            }
+            *d = n;
           } else {
-            const R a0 = abs_sq<R>(n0);
-            const R a1 = abs_sq<R>(n1);
-            local_max = a0 > local_max ? a0 : local_max;
-            local_max = a1 > local_max ? a1 : local_max;
+            const C g0 = work[r * PLS + 2 * col];
+            const C g1 = work[r * PLS + 2 * col + 1];
+            float4 *d4 = reinterpret_cast<float4 *>(dst) + r * CW + col;
+            if (!need_x) {
+              *d4 = make_float4((float)g0.x, (float)g0.y, (float)g1.x, (float)g1.y);
+              continue;
+            }
+            C n0 = cmake<C>(sub_rn<R>((R)xv[j].x, mul_rn<R>(step, g0.x)),
+                            sub_rn<R>((R)xv[j].y, mul_rn<R>(step, g0.y)));
+            C n1 = cmake<C>(sub_rn<R>((R)xv[j].z, mul_rn<R>(step, g1.x)),
+                            sub_rn<R>((R)xv[j].w, mul_rn<R>(step, g1.y)));
+            if (epilogue == kUpdateThreshold) {
+              n0 = soft_threshold<R>(n0, lamb, lamb_sq);
+              n1 = soft_threshold<R>(n1, lamb, lamb_sq);
+            } else {
+              const R a0 = abs_sq<R>(n0);
+              const R a1 = abs_sq<R>(n1);
+              local_max = a0 > local_max ? a0 : local_max;
+              local_max = a1 > local_max ? a1 : local_max;
+            }
+            *d4 = make_float4((float)n0.x, (float)n0.y, (float)n1.x, (float)n1.y);
           }
-          *d4 = make_float4((float)n0.x, (float)n0.y, (float)n1.x, (float)n1.y);
         }
       }
     } else {
