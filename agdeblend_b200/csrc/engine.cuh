@@ -775,6 +775,10 @@ class Engine {
         add_fwd_rows<1, 40, 1, 1, 256, 64, 2>(c);
         add_adj_rows<1, 40, 1, 1, 256, 64, 2, 2>(c);
         add_adj_pipe<1, 40, 1, 1, 256, 128, 2>(c);
+        add_fwd<1, 40, 1, 1, 64, 64, 1, 6>(c);
+        add_fwd<1, 40, 1, 1, 128, 128, 1, 4>(c);
+        add_adj_pipe<1, 40, 1, 1, 64, 64, 6>(c);
+        add_adj_pipe<1, 40, 1, 1, 128, 96, 4>(c);
       } else if (shape_is<1, 20, 1, 1>(W)) {
         add_fwd<1, 20, 1, 1, 256, 256, 2, 1>(c);
         add_fwd<1, 20, 1, 1, 256, 128, 1, 3>(c);
@@ -786,6 +790,10 @@ class Engine {
         add_adj_rows<1, 20, 1, 1, 256, 128, 2, 2>(c);
         add_adj_pipe<1, 20, 1, 1, 256, 160, 3>(c);
         add_adj_pipe<1, 20, 1, 1, 256, 256, 2>(c);
+        add_fwd<1, 20, 1, 1, 64, 64, 1, 12>(c);
+        add_fwd<1, 20, 1, 1, 128, 128, 1, 6>(c);
+        add_adj_pipe<1, 20, 1, 1, 64, 64, 10>(c);
+        add_adj_pipe<1, 20, 1, 1, 128, 128, 5>(c);
       } else if (shape_is<2, 20, 40, 1>(W)) {
         add_fwd<2, 20, 40, 1, 384, 16, 2, 1>(c);
         add_fwd<2, 20, 40, 1, 256, 12, 1, 2>(c);
@@ -811,6 +819,9 @@ class Engine {
         add_adj_rows<2, 20, 20, 1, 256, 10, 2, 2>(c);
         add_adj_pipe<2, 20, 20, 1, 256, 12, 3>(c);
         add_adj_pipe<2, 20, 20, 1, 256, 16, 2>(c);
+        add_fwd<2, 20, 20, 1, 128, 6, 1, 6>(c);
+        add_adj_pipe<2, 20, 20, 1, 64, 4, 8>(c);
+        add_adj_pipe<2, 20, 20, 1, 128, 8, 4>(c);
         add_adj_pipe<2, 20, 20, 1, 256, 8, 2, true>(c);
       } else if (shape_is<2, 40, 40, 1>(W)) {
         add_fwd<2, 40, 40, 1, 320, 8, 2, 1>(c);
@@ -822,6 +833,8 @@ class Engine {
         add_fwd_rows<2, 40, 40, 1, 256, 4, 2>(c);
         add_adj_rows<2, 40, 40, 1, 256, 3, 2, 2>(c);
         add_adj_pipe<2, 40, 40, 1, 256, 4, 2>(c);
+        add_adj_pipe<2, 40, 40, 1, 128, 2, 4>(c);
+        add_adj_pipe<2, 40, 40, 1, 64, 1, 8>(c);
       } else if (shape_is<3, 20, 20, 20>(W)) {
         add_fwd<3, 20, 20, 20, 512, 1, 2, 1>(c);
         add_fwd<3, 20, 20, 20, 256, 1, 1, 3>(c);
