@@ -542,6 +542,18 @@ __global__ void __launch_bounds__(NT, (sizeof(R) == sizeof(float) ? 512 : 384) /
       tab_b = b.tab;
     }
     const C *src = job.src + l0 * b.n_in;
+    if (threadIdx.x == 0) {
+      // into L2: the model lines that the update will read, and the next
+      // batch's lines
+      if (!FWD && epilogue != kStore)
+        prefetch_l2(job.dst + l0 * b.n_out, n * b.n_out * (long)sizeof(C));
+      if (bi + gridDim.x < n_batch) {
+        const PlaneDftJob<R> &nj = jobs[batch_job[bi + gridDim.x]];
+        const long m0 = batch_line[bi + gridDim.x];
+        prefetch_l2(nj.src + m0 * nj.b.n_in,
+                    min((long)nj.np, nj.planes - m0) * nj.b.n_in * (long)sizeof(C));
+      }
+    }
     const int cpr = min(b.n_in, NT);
     const int tr = NT / cpr;
     const int r0 = threadIdx.x / cpr;
