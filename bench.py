@@ -411,16 +411,12 @@ def measure_single(args, name, rank, world, local, cpu_its):
     # time kernel reads the residual; the time-axis kernels move only
     # intermediates (0 algorithmic bytes).
     nf = int(prof[14])
-    fast = int(info[8]) == 1
     wav = sv.wavelets is not None
-    wav_fast = int(info[9]) == 1
     # phases named by the kernel family the set-up picked for them
-    names = ((kn["space_fwd"], kn["time_fwd"], "blend_gather", kn["time_adj"], kn["space_adj"])
-             if fast else
-             ("axis_pass_fwd0", "time_c2r_ola", "blend_gather", "time_r2c", "axis_pass_adj_last"))
+    names = (kn["space_fwd"], kn["time_fwd"], "record_gather", kn["time_adj"], kn["space_adj"])
     if wav:
         # the adjoint time phase then also holds the wavelet correlation
-        names = names[:3] + (names[3] + "+" + ("wavelet_fast" if wav_fast else "wavelet_apply"),
+        names = names[:3] + (names[3] + "+" + kn["wavelet"],
                              names[4])
     phases = {
         names[0]: (prof[6], 8.0 * M),
@@ -430,7 +426,7 @@ def measure_single(args, name, rank, world, local, cpu_its):
         names[4]: (prof[10 + nf - 1], 16.0 * M),
     }
     if wav:
-        phases["wavelet_fast" if wav_fast else "wavelet_apply"] = (prof[2], 0.0)
+        phases[kn["wavelet"]] = (prof[2], 0.0)
     dom = max(phases, key=lambda k: phases[k][0])
     dom_ms, dom_bytes = phases[dom]
     iter_bytes = 3 * 8.0 * M + 4 * 4.0 * Rn
