@@ -868,7 +868,7 @@ class Engine {
         add_fwd<2, 20, 40, 1, 64, 3, 1, 4>(c);
         add_adj_pipe<2, 20, 40, 1, 128, 4, 2>(c);
         add_adj_pipe<2, 20, 40, 1, 64, 2, 4>(c);
-        add_adj_pipe<2, 20, 40, 1, 80, 2, 3>(c);
+        add_adj_pipe<2, 20, 40, 1, 96, 2, 3>(c);
       } else if (shape_is<2, 20, 20, 1>(W)) {
         add_fwd<2, 20, 20, 1, 384, 12, 2, 1>(c);
         add_adj<2, 20, 20, 1, 384, 10, 2, 1>(c);

@@ -625,6 +625,7 @@ template <typename R, int D, int P0, int P1, int P2, int NT, int NP, int STAGES,
 __global__ void __launch_bounds__(NT, MINB)
     space_adj_fast(PlaneBatches<R> batches, int epilogue, R step_arg, R lamb_arg,
                    const R *step_dev, const R *lamb_dev, R *max_out) {
+  static_assert(NT % 32 == 0, "block_max needs whole warps");
   static_assert(STAGES == 1 || STAGES == 2, "one or two stages");
   using C = Cx<R>;
   using S = PlaneShape<D, P0, P1, P2>;
@@ -833,6 +834,7 @@ template <typename R, int D, int P0, int P1, int P2, int NT, int NP, int STAGES,
 __global__ void __launch_bounds__(NT, MINB)
     space_adj_rows(PlaneBatches<R> batches, int epilogue, R step_arg, R lamb_arg,
                    const R *step_dev, const R *lamb_dev, R *max_out) {
+  static_assert(NT % 32 == 0, "block_max needs whole warps");
   static_assert(STAGES == 1 || STAGES == 2, "one or two stages");
   using C = Cx<R>;
   using S = PlaneShape<D, P0, P1, P2>;
@@ -1006,6 +1008,7 @@ __global__ void __launch_bounds__(NT, MINB)
   constexpr int PL = S::PL;
   constexpr int PLS = S::PLS;
   constexpr int ROWS = S::dense_P / PL;
+  static_assert(NT % 32 == 0, "block_max needs whole warps");
   static_assert(Z == ROWS * PLS, "padded rows evenly spaced");
   constexpr int EV = sizeof(C) == 8 ? 2 : 1;  // values of a 16-byte column
   using Col = typename std::conditional<EV == 2, float4, C>::type;

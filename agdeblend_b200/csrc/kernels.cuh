@@ -155,6 +155,9 @@ __device__ __forceinline__ void atomic_max_nonneg(double *addr, double v) {
             (unsigned long long)__double_as_longlong(v));
 }
 
+// Largest value (sum) of the block, in its first warp.  Blocks of whole warps
+// only: a partial warp would be left out of the second stage, and its
+// shuffles would name lanes that do not exist.
 template <typename R>
 __device__ R block_max(R v, R *red) {
   for (int o = 16; o > 0; o >>= 1) {
