@@ -34,12 +34,16 @@ static void check(cudaError_t e, const char *what) {
 // the work of their engine's stream that used them has been waited for, so
 // no kernel can still use them.  A block belongs to the device it was
 // allocated on, whichever device is current when it comes back.  Sizes are
-// rounded up to kGrain.  Best fit within a factor of two; at most half the
-// device memory is held (AGD_GPU_CACHE=0 disables the cache;
-// agd_gpu_release_cache frees it).
+// rounded up to kGrain; a request takes the smallest block that fits if that
+// is at most twice as large (from kLarge on, twice and kSlack more), so that
+// tables leave the blocks of large arrays alone.  At most half the device
+// memory is held (AGD_GPU_CACHE=0 disables the cache; agd_gpu_release_cache
+// frees it).
 class DevicePool {
  public:
   static constexpr size_t kGrain = 512;
+  static constexpr size_t kLarge = size_t(1) << 16;
+  static constexpr size_t kSlack = size_t(1) << 20;
 
   static void *take(size_t bytes) {
     bytes = (bytes + kGrain - 1) / kGrain * kGrain;
@@ -50,7 +54,7 @@ class DevicePool {
       std::lock_guard<std::mutex> g(mu());
       auto &m = free_blocks()[dev];
       auto it = m.lower_bound(bytes);
-      if (it != m.end() && it->first <= 2 * bytes + (size_t(1) << 20)) {
+      if (it != m.end() && it->first <= 2 * bytes + (bytes >= kLarge ? kSlack : 0)) {
         void *p = it->second;
         held() -= it->first;
         m.erase(it);

@@ -1,7 +1,7 @@
 """The cache of device blocks (agdeblend_b200/csrc/device_pool.hpp), compiled for
 the host against the CUDA headers and a fake of the runtime calls it makes
 (addresses count up, each remembers its device): a block goes back to the
-device it was allocated on."""
+device it was allocated on; a table does not take the block of a large array."""
 import os
 import shutil
 import subprocess
@@ -67,12 +67,25 @@ static int device_of_a_block() {
   return g_frees == 2 && g_dev == 0 ? 0 : 3;
 }
 
+static int large_blocks_are_left_to_large_arrays() {
+  DevArray<char> big;
+  big.alloc(1 << 20);
+  void *block = big.get();
+  big.release();
+  DevArray<char> table, again;
+  table.alloc(512);
+  if (table.get() == block) return 1;
+  again.alloc(900000);
+  return again.get() == block ? 0 : 2;
+}
+
 int main(int, char **argv) {
-  int (*const cases[])() = {device_of_a_block};
+  int (*const cases[])() = {device_of_a_block, large_blocks_are_left_to_large_arrays};
   return cases[std::atoi(argv[1])]();
 }
 """
-CASES = ["device_of_a_block"]
+CASES = ["device_of_a_block",
+         "large_blocks_are_left_to_large_arrays"]
 
 
 @pytest.fixture(scope="module")
