@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <cstdio>
 #include <cstdlib>
+#include <exception>
 #include <map>
 #include <mutex>
 #include <stdexcept>
@@ -31,8 +32,8 @@ static void check(cudaError_t e, const char *what) {
 // cudaMalloc of gigabytes costs page mapping that can exceed the solve
 // itself, and the fifty small tables of a 40-trace gather cost 0.3 ms of a
 // 1.1 ms call in cudaMalloc and cudaFree.  Blocks enter the cache only when
-// the work of their engine's stream that used them has been waited for, so
-// no kernel can still use them.  A block belongs to the device it was
+// their engine has waited for the work that used them, so no kernel can
+// still use them; a block that an exception releases is freed instead.  A block belongs to the device it was
 // allocated on, whichever device is current when it comes back.  Sizes are
 // rounded up to kGrain; a request takes the smallest block that fits if that
 // is at most twice as large (from kLarge on, twice and kSlack more), so that
@@ -78,7 +79,10 @@ class DevicePool {
     if (p == nullptr) return;
     std::lock_guard<std::mutex> g(mu());
     const Block b = blocks()[p];
-    if (!enabled() || held() + b.bytes > half_memory(b.dev)) {
+    // released by an exception: launches before it may still use the block,
+    // and cudaFree waits for the device
+    if (std::uncaught_exceptions() > 0 || !enabled() ||
+        held() + b.bytes > half_memory(b.dev)) {
       blocks().erase(p);
       cudaFree(p);
       return;
@@ -182,9 +186,9 @@ class DevArray {
     return *this;
   }
   ~DevArray() { release(); }
-  // From the device cache; when the array is released, the work on its
-  // engine's stream that uses it must have been waited for (engine members:
-  // the engine synchronises before destruction).
+  // From the device cache; when the array is released (other than by an
+  // exception), the work on its engine's stream that uses it must have been
+  // waited for (engine members: the engine synchronises before destruction).
   void alloc(size_t n) {
     release();
     if (n) p_ = static_cast<T *>(DevicePool::take(n * sizeof(T)));

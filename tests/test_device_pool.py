@@ -1,7 +1,8 @@
 """The cache of device blocks (agdeblend_b200/csrc/device_pool.hpp), compiled for
 the host against the CUDA headers and a fake of the runtime calls it makes
 (addresses count up, each remembers its device): a block goes back to the
-device it was allocated on; a table does not take the block of a large array."""
+device it was allocated on; a table does not take the block of a large array;
+a block that an exception releases is freed (cudaFree waits for the device)."""
 import os
 import shutil
 import subprocess
@@ -79,13 +80,24 @@ static int large_blocks_are_left_to_large_arrays() {
   return again.get() == block ? 0 : 2;
 }
 
+static int exceptions_free_their_blocks() {
+  try {
+    DevArray<char> tmp;
+    tmp.alloc(3000000);
+    throw 1;
+  } catch (int) {
+  }
+  return g_frees == 1 ? 0 : 1;
+}
+
 int main(int, char **argv) {
-  int (*const cases[])() = {device_of_a_block, large_blocks_are_left_to_large_arrays};
+  int (*const cases[])() = {device_of_a_block, large_blocks_are_left_to_large_arrays, exceptions_free_their_blocks};
   return cases[std::atoi(argv[1])]();
 }
 """
 CASES = ["device_of_a_block",
-         "large_blocks_are_left_to_large_arrays"]
+         "large_blocks_are_left_to_large_arrays",
+         "exceptions_free_their_blocks"]
 
 
 @pytest.fixture(scope="module")
