@@ -736,6 +736,7 @@ __global__ void record_sumsq(const R *__restrict__ x, long n, double *out) {
 // The schedule step alone, for problems without a record.
 template <typename R>
 __global__ void next_lambda(NextLambda<R> lambda) {
+  pdl_enter();
   lambda.advance();
 }
 
