@@ -17,8 +17,9 @@ def _kernels(header):
     with open(os.path.join(CSRC, header)) as f:
         text = f.read()
     out = {}
-    for m in re.finditer(r"__global__ void\s*(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\))?"
-                         r"\s*(\w+)\([^{;]*\)\s*\{", text):
+    nested = r"\((?:[^()]|\((?:[^()]|\([^()]*\))*\))*\)"  # parentheses, three deep
+    for m in re.finditer(rf"__global__ void\s+(?:__launch_bounds__{nested}\s*)?"
+                         r"(\w+)\([^{;]*\)\s*\{", text):
         depth, end = 1, m.end()
         while depth:
             depth += {"{": 1, "}": -1}.get(text[end], 0)
