@@ -224,20 +224,13 @@ class Engine {
   // own static shared memory; smem_max becomes the smallest such limit.
   template <typename K>
   int opt_in(K kernel, int limit) {
-    // once per kernel and device: the attribute stays
-    static std::mutex mu;
-    static std::map<std::pair<int, const void *>, int> done;
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
-    const std::pair<int, const void *> key(dev, reinterpret_cast<const void *>(kernel));
-    std::lock_guard<std::mutex> lk(mu);
-    const auto it = done.find(key);
-    if (it != done.end()) return it->second;
+    // set once per kernel and context: the attribute stays, and is asked for
+    // in the context itself, which a device reset replaces
     cudaFuncAttributes fa;
     CK(cudaFuncGetAttributes(&fa, kernel));
     const int dyn = limit - (int)fa.sharedSizeBytes;
-    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-    done[key] = dyn;
+    if (fa.maxDynamicSharedSizeBytes != dyn)
+      CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
     return dyn;
   }
 
@@ -270,14 +263,16 @@ class Engine {
   }
 
   // twiddle tables of the register DFTs in constant memory of the current
-  // device (fast.cuh), shared by the fast space, time and wavelet kernels
+  // context (fast.cuh), shared by the fast space, time and wavelet kernels;
+  // filled once per context, which tables_mark's attribute tells (a device
+  // reset clears both)
   void upload_twiddles() {
+    constexpr int kFilled = 65536;  // above the 48 KB that a kernel starts with
     static std::mutex mu;
-    static std::map<int, bool> done;  // per device: the tables stay
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(mu);
-    if (done[dev]) return;
+    cudaFuncAttributes fa;
+    CK(cudaFuncGetAttributes(&fa, tables_mark<R>));
+    if (fa.maxDynamicSharedSizeBytes == kFilled) return;
     std::vector<C> tw(kTwTotal);
     for (int i = 0, off = 0; i < kNumTw; off += kTwSizes[i], ++i)
       for (int k = 0; k < kTwSizes[i]; ++k) {
@@ -292,7 +287,8 @@ class Engine {
       CK(cudaMemcpyToSymbolAsync(c_tw_d, tw.data(), tw.size() * sizeof(C), 0,
                                  cudaMemcpyHostToDevice, stream));
     CK(cudaStreamSynchronize(stream));
-    done[dev] = true;
+    CK(cudaFuncSetAttribute(tables_mark<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            kFilled));
   }
 
   // C = product of pairwise coprime prime powers with a register DFT; the

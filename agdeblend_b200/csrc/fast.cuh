@@ -55,6 +55,10 @@ constexpr int kTwTotal = tw_total();
 static __constant__ float2 c_tw_f[kTwTotal];
 static __constant__ double2 c_tw_d[kTwTotal];
 
+// Never launched: an attribute of it marks a context whose tables are filled.
+template <typename R>
+__global__ void tables_mark() {}
+
 template <typename R>
 __device__ __forceinline__ Cx<R> ctw(int idx);
 template <>
