@@ -24,6 +24,14 @@
 //    f32x2 multiply-adds on the (re, im) pairs: the same rate as scalar
 //    ones at half the issue slots); eight threads share the table values,
 //    so the shared memory delivers half of what it could;
+//  * one running sum of P / 2 terms loses more than the stages of radix
+//    passes do where P is composite (relative L2 error of the operators on
+//    80 x 80 planes 1.19 times theirs, on 44 x 44 1.06).  Such axes sum in
+//    runs of four or eight terms whose sums are then added up; the totals
+//    take the registers of half the tile's lines (2 lines x 4 output pairs).
+//    0.98 and 0.97 times the radix passes' error then, at 1.2 times the time
+//    of one sum (planes of 60 x 60, 28.9 M values: forward 320 -> 364 us,
+//    adjoint 370 -> 433; radix passes 718 and 873);
 //  * the raw planes of the next batch are copied (cp.async) into a staging
 //    buffer behind the products of this one; a thread forms the pairs s, d
 //    as it reads the lines, and the contiguous axis is transformed in place,
@@ -56,6 +64,7 @@ template <typename R>
 struct DftAxis {
   const R *tab;
   int P, H, kpad, n_in, n_out;
+  int run;  // terms summed before they are added to the total (0: one sum)
 };
 
 // One window's planes: rows along axis b (contiguous), columns along axis a
@@ -85,6 +94,10 @@ struct AxisDftJob {
 // output pairs per thread: registers for 4 x 4 packed floats, 4 x 2 doubles
 template <typename R>
 constexpr int kDftTk = sizeof(R) == sizeof(float) ? 4 : 2;
+
+// lines per thread's tile: 4, or 2 where the sums run in two levels, whose
+// totals take the registers of the other two lines
+__host__ __device__ inline int dft_tile_lines(int run) { return run > 0 ? 2 : 4; }
 
 __host__ __device__ inline int dft_round4(int n) { return (n + 3) & ~3; }
 
@@ -181,24 +194,28 @@ __device__ __forceinline__ void dft_load_table(R *to, const DftAxis<R> &x) {
   for (int e = threadIdx.x; e < n; e += NT) cp_async<16>(to + e * per, x.tab + e * per);
 }
 
-// Accumulators of a tile of 4 lines x TK output pairs.
-template <typename R>
+// Accumulators of a tile of TL lines x TK output pairs; with TL = 2, the
+// totals of the runs before this one.
+template <typename R, int TL>
 struct DftTile {
   static constexpr int TK = kDftTk<R>;
-  Cx<R> a[4][TK], b[4][TK];
+  static constexpr bool kTwo = TL == 2;
+  Cx<R> a[TL][TK], b[TL][TK];
+  Cx<R> ta[kTwo ? TL : 1][TK], tb[kTwo ? TL : 1][TK];
 
   // from x_0 and x_{P/2} (k0 is even: the sign of x_{P/2} follows m)
-  __device__ __forceinline__ void start(const Cx<R> (&u)[4], const Cx<R> (&v)[4]) {
+  __device__ __forceinline__ void start(const Cx<R> (&u)[TL], const Cx<R> (&v)[TL]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < TL; ++i)
 #pragma unroll
       for (int m = 0; m < TK; ++m) {
         a[i][m] = (m & 1) ? csub(u[i], v[i]) : cadd(u[i], v[i]);
         b[i][m] = cmake<Cx<R>>((R)0, (R)0);
+        if constexpr (kTwo) ta[i][m] = tb[i][m] = b[i][m];
       }
   }
   // one pair (s, d) of each line, with the table values at c, n
-  __device__ __forceinline__ void add(const Cx<R> (&s)[4], const Cx<R> (&d)[4], const R *c,
+  __device__ __forceinline__ void add(const Cx<R> (&s)[TL], const Cx<R> (&d)[TL], const R *c,
                                       const R *n) {
     R cv[TK], nv[TK];
     load_tab(c, cv);
@@ -206,9 +223,34 @@ struct DftTile {
 #pragma unroll
     for (int m = 0; m < TK; ++m)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < TL; ++i) {
         fma_real(a[i][m], s[i], cv[m]);
         fma_real(b[i][m], d[i], nv[m]);
+      }
+  }
+  // the same as the first pair of a run: the last run's sums go to the totals
+  __device__ __forceinline__ void add_new_run(const Cx<R> (&s)[TL], const Cx<R> (&d)[TL],
+                                              const R *c, const R *n) {
+    R cv[TK], nv[TK];
+    load_tab(c, cv);
+    load_tab(n, nv);
+#pragma unroll
+    for (int m = 0; m < TK; ++m)
+#pragma unroll
+      for (int i = 0; i < TL; ++i) {
+        ta[i][m] = cadd(ta[i][m], a[i][m]);
+        tb[i][m] = cadd(tb[i][m], b[i][m]);
+        a[i][m] = cscale(s[i], cv[m]);
+        b[i][m] = cscale(d[i], nv[m]);
+      }
+  }
+  __device__ __forceinline__ void finish() {
+#pragma unroll
+    for (int i = 0; i < TL; ++i)
+#pragma unroll
+      for (int m = 0; m < TK; ++m) {
+        a[i][m] = cadd(ta[i][m], a[i][m]);
+        b[i][m] = cadd(tb[i][m], b[i][m]);
       }
   }
   // outputs k0 .. of line i at out + k * ks, k < n_out
@@ -231,16 +273,17 @@ struct DftTile {
 };
 
 // The thread's tile number -> line tile and output tile: blocks of eight
-// line tiles (fewer in the last), in a block output tile by output tile.
-// Lines of the tile: l0 + i * step with w the block's line tiles.
+// line tiles of tl lines (fewer in the last), in a block output tile by
+// output tile.  Lines of the tile: line0 + at + i * w with w the block's line
+// tiles.
 struct DftTileAt {
   int line0, w, k;
-  __device__ __forceinline__ DftTileAt(int tile, int lt_n, int kt_n) {
+  __device__ __forceinline__ DftTileAt(int tile, int lt_n, int kt_n, int tl) {
     const int blk = tile / (8 * kt_n);
     const int rem = tile - blk * 8 * kt_n;
     w = min(8, lt_n - 8 * blk);
     k = rem / w;
-    line0 = 32 * blk;
+    line0 = 8 * tl * blk;
     at = rem - k * w;
   }
   int at;
@@ -248,63 +291,116 @@ struct DftTileAt {
 
 // Accumulates a tile from raw lines in shared memory: element e of line i at
 // lo[i] + e * es, zero from n_in on.
-template <typename R>
-__device__ __forceinline__ void dft_accumulate_raw(DftTile<R> &acc, const Cx<R> *const (&lo)[4],
-                                                   int es, const DftAxis<R> &x, const R *tab,
-                                                   int k0) {
+template <typename R, int TL>
+__device__ __forceinline__ void dft_accumulate_raw(DftTile<R, TL> &acc,
+                                                   const Cx<R> *const (&lo)[TL], int es,
+                                                   const DftAxis<R> &x, const R *tab, int k0) {
   using C = Cx<R>;
+  constexpr bool kTwo = TL == 2;
   const int mid = x.P / 2;
   const bool has_mid = x.P % 2 == 0 && mid < x.n_in;
   const int both = min(x.P - x.n_in, x.H);  // pairs 1 .. both have one member
-  C u[4], v[4];
+  C u[TL], v[TL];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < TL; ++i) {
     u[i] = lo[i][0];
     v[i] = has_mid ? lo[i][mid * es] : cmake<C>((R)0, (R)0);
   }
   acc.start(u, v);
   const R *cj = tab + k0;
   const R *nj = cj + x.H * x.kpad;
-  int j = 1, e = es;
-#pragma unroll 1
-  for (; j <= both; ++j, e += es, cj += x.kpad, nj += x.kpad) {
+  int j = 1, e = es, f = (x.P - 1) * es;
+  // one pair of each line: elements e and, with both members present, f
+  auto term = [&](bool both_in, bool new_run) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) u[i] = lo[i][e];
-    acc.add(u, u, cj, nj);
-  }
-  int f = (x.P - j) * es;
+    for (int i = 0; i < TL; ++i) {
+      if (both_in)
+        sum_diff(lo[i][e], lo[i][f], u[i], v[i]);
+      else
+        u[i] = v[i] = lo[i][e];
+    }
+    if constexpr (kTwo) {
+      if (new_run)
+        acc.add_new_run(u, v, cj, nj);
+      else
+        acc.add(u, v, cj, nj);
+    } else {
+      acc.add(u, v, cj, nj);
+    }
+    ++j;
+    e += es;
+    f -= es;
+    cj += x.kpad;
+    nj += x.kpad;
+  };
+  if constexpr (kTwo) {
+    // the pairs with one member, then those with both, in runs
+    int end = x.run;  // last pair of the run
+    bool fresh = false;
+    while (j <= both) {
+      const int stop = min(both, end);
+      term(false, fresh);
+      fresh = false;
+#pragma unroll 2
+      while (j <= stop) term(false, false);
+      if (j > end) {
+        end += x.run;
+        fresh = true;
+      }
+    }
+    while (j <= x.H) {
+      const int stop = min(x.H, end);
+      term(true, fresh);
+      fresh = false;
+#pragma unroll 2
+      while (j <= stop) term(true, false);
+      if (j > end) {
+        end += x.run;
+        fresh = true;
+      }
+    }
+    acc.finish();
+  } else {
 #pragma unroll 1
-  for (; j <= x.H; ++j, e += es, f -= es, cj += x.kpad, nj += x.kpad) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) sum_diff(lo[i][e], lo[i][f], u[i], v[i]);
-    acc.add(u, v, cj, nj);
+    while (j <= both) term(false, false);
+#pragma unroll 1
+    while (j <= x.H) term(true, false);
   }
 }
 
 // All outputs of n_lines raw lines in shared memory: element e of line q at
 // raw + in_at(q) + e * es; outputs to out_at(q) + k * ks.  Lines past n_lines
 // take the last line's place and are not stored.
-template <typename R, bool FWD, typename InAt, typename OutAt, typename I>
-__device__ __forceinline__ void dft_from_raw(const Cx<R> *raw, int es, int n_lines,
-                                             const DftAxis<R> &x, const R *tab, InAt in_at,
-                                             OutAt out_at, I ks) {
+template <typename R, bool FWD, int TL, typename InAt, typename OutAt, typename I>
+__device__ __forceinline__ void dft_tiles_from_raw(const Cx<R> *raw, int es, int n_lines,
+                                                   const DftAxis<R> &x, const R *tab, InAt in_at,
+                                                   OutAt out_at, I ks) {
   const int kt_n = x.kpad / kDftTk<R>;
-  const int lt_n = (n_lines + 3) / 4;
+  const int lt_n = (n_lines + TL - 1) / TL;
   for (int tile = threadIdx.x; tile < lt_n * kt_n; tile += kDftThreads) {
-    const DftTileAt t(tile, lt_n, kt_n);
+    const DftTileAt t(tile, lt_n, kt_n, TL);
     const int k0 = kDftTk<R> * t.k;
-    const Cx<R> *lo[4];
+    const Cx<R> *lo[TL];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < TL; ++i)
       lo[i] = raw + in_at(min(t.line0 + t.at + i * t.w, n_lines - 1));
-    DftTile<R> acc;
-    dft_accumulate_raw<R>(acc, lo, es, x, tab, k0);
+    DftTile<R, TL> acc;
+    dft_accumulate_raw<R, TL>(acc, lo, es, x, tab, k0);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < TL; ++i) {
       const int q = t.line0 + t.at + i * t.w;
       if (q < n_lines) acc.template store<FWD>(i, out_at(q), ks, k0, x);
     }
   }
+}
+template <typename R, bool FWD, typename InAt, typename OutAt, typename I>
+__device__ __forceinline__ void dft_from_raw(const Cx<R> *raw, int es, int n_lines,
+                                             const DftAxis<R> &x, const R *tab, InAt in_at,
+                                             OutAt out_at, I ks) {
+  if (x.run > 0)
+    dft_tiles_from_raw<R, FWD, 2>(raw, es, n_lines, x, tab, in_at, out_at, ks);
+  else
+    dft_tiles_from_raw<R, FWD, 4>(raw, es, n_lines, x, tab, in_at, out_at, ks);
 }
 
 // The transforms of n rows of shared memory (elements side by side, rows rs
@@ -312,33 +408,41 @@ __device__ __forceinline__ void dft_from_raw(const Cx<R> *raw, int es, int n_lin
 // for, all read before any is overwritten.  Every warp meets the block's
 // barrier once per step, with tiles or without (the two places are separate
 // so that the accumulators need no values in idle warps).
-template <typename R, bool FWD, int NT>
-__device__ __forceinline__ void dft_rows_in_place(Cx<R> *rows, int rs, int n,
-                                                  const DftAxis<R> &x, const R *tab) {
+template <typename R, bool FWD, int NT, int TL>
+__device__ __forceinline__ void dft_tiles_in_place(Cx<R> *rows, int rs, int n,
+                                                   const DftAxis<R> &x, const R *tab) {
   const int kt_n = x.kpad / kDftTk<R>;
-  const int per = 4 * (NT / kt_n);
+  const int per = TL * (NT / kt_n);
   for (int r0 = 0; r0 < n; r0 += per, rows += per * rs) {
     const int m = min(per, n - r0);
-    const int lt_n = (m + 3) / 4;
+    const int lt_n = (m + TL - 1) / TL;
     const int tiles = lt_n * kt_n;
     if ((int)(threadIdx.x & ~31) >= tiles) {  // a warp without tiles
       asm volatile("barrier.sync 0;" ::: "memory");
       continue;
     }
-    const DftTileAt t(min((int)threadIdx.x, tiles - 1), lt_n, kt_n);
+    const DftTileAt t(min((int)threadIdx.x, tiles - 1), lt_n, kt_n, TL);
     const int k0 = kDftTk<R> * t.k;
-    DftTile<R> acc;
-    const Cx<R> *lo[4];
+    DftTile<R, TL> acc;
+    const Cx<R> *lo[TL];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) lo[i] = rows + min(t.line0 + t.at + i * t.w, m - 1) * rs;
-    dft_accumulate_raw<R>(acc, lo, 1, x, tab, k0);
+    for (int i = 0; i < TL; ++i) lo[i] = rows + min(t.line0 + t.at + i * t.w, m - 1) * rs;
+    dft_accumulate_raw<R, TL>(acc, lo, 1, x, tab, k0);
     asm volatile("barrier.sync 0;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < TL; ++i) {
       const int q = t.line0 + t.at + i * t.w;
       if ((int)threadIdx.x < tiles && q < m) acc.template store<FWD>(i, rows + q * rs, 1, k0, x);
     }
   }
+}
+template <typename R, bool FWD, int NT>
+__device__ __forceinline__ void dft_rows_in_place(Cx<R> *rows, int rs, int n,
+                                                  const DftAxis<R> &x, const R *tab) {
+  if (x.run > 0)
+    dft_tiles_in_place<R, FWD, NT, 2>(rows, rs, n, x, tab);
+  else
+    dft_tiles_in_place<R, FWD, NT, 4>(rows, rs, n, x, tab);
 }
 
 // Finished rows of shared memory (stride rs) to n rows of n_out values at
