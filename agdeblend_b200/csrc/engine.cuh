@@ -1160,11 +1160,14 @@ class Engine {
   // Planes per batch of every job: the number with the least warp work per
   // plane (whole warps of 4-line tiles; the constant stands for a batch's
   // barriers and first loads), within a block's share of the shared memory
-  // and small enough that the batches fill the device.
+  // and small enough that the batches fill the device.  The smallest planes
+  // take the most: 3 x 3, 47.5 M values, forward and adjoint together 2352 us
+  // in batches of 32, 831 in 128 (5 x 5, 32.1 M: 728 and 389, 497 in 256);
+  // radix passes 1481 and 953.
   void pick_plane_batches(std::vector<PlaneDftJob<R>> &jobs) const {
     long total = 0;
     for (const auto &j : jobs) total += j.planes;
-    const long most = std::min<long>(32, std::max<long>(1, total / (4L * n_sm)));
+    const long most = std::min<long>(128, std::max<long>(1, total / (4L * n_sm)));
     for (auto &j : jobs) {
       double best = 1e300;
       j.np = 1;

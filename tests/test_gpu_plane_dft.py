@@ -135,3 +135,32 @@ def test_no_less_accurate_than_the_radix_passes(length):
         p.close()
     for table, radix in zip(*errors):
         assert table <= 1.01 * radix
+
+
+def _space_ms(sv, dtype, generic):
+    """Space phases (forward and adjoint) of an iteration, the fastest of eight."""
+    old = os.environ.get("AGD_GPU_GENERIC")
+    os.environ["AGD_GPU_GENERIC"] = "1" if generic else "0"
+    try:
+        p = A.Problem.from_survey(sv, dtype)
+    finally:
+        if old is None:
+            os.environ.pop("AGD_GPU_GENERIC", None)
+        else:
+            os.environ["AGD_GPU_GENERIC"] = old
+    p.time_iterations(sv.data, 1.0, sv.n_its, 2, 4)
+    ms = min(t[0] + t[5] for t in (p.profile_iteration(1e-3) for _ in range(8)))
+    p.close()
+    return ms
+
+
+# space shape, windows, type: padded 3 x 3
+SPEED = [((60, 60), (2, 2), np.float32), ((60, 60), (2, 2), np.float64)]
+
+
+@pytest.mark.parametrize("space,windows,dtype", SPEED)
+def test_not_slower_than_the_radix_passes(space, windows, dtype):
+    """A shape goes to the table DFTs only where they are faster (1.1: the
+    spread of the timing where both sides are the same kernels)."""
+    sv = _survey(space, windows, nt=600, wt=128)
+    assert _space_ms(sv, dtype, False) <= 1.1 * _space_ms(sv, dtype, True)
