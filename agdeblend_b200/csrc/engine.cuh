@@ -966,7 +966,11 @@ class Engine {
       classes[k]->win.push_back(w);
     }
     // any other shape up to kDftMaxP per axis: table-DFT kernels, with the
-    // last two axes in one kernel when a plane of them fits in shared memory
+    // last two axes in one kernel when a plane of them takes at most a third
+    // of an SM's shared memory.  A block's waits are covered by the other
+    // blocks only: planes of 80 x 80 (one block per SM) 875 us forward and
+    // adjoint, as two passes 594; 75 x 75 (two) 660 and 514; 60 x 60 (three)
+    // 798 and 769.
     win_dft.assign(nw, 0);
     for (int w = 0; w < nw && !generic_only; ++w) {
       const WindowPlan &W = plan.windows[w];
@@ -974,13 +978,13 @@ class Engine {
       bool ok = true, plane = W.D > 1;
       for (int d = 0; d < W.D; ++d) ok = ok && W.P[d] >= 3 && W.P[d] <= kDftMaxP;
       if (!ok) continue;
+      const size_t third = (size_t)(sm_smem / 3 - 2 * block_reserved);
       for (bool fwd : {true, false}) {
         const DftAxis<R> b = dft_axis(W, W.D - 1, fwd);
         ok = ok && line_dft_smem<R>(b, 4) <= (size_t)smem_max;
         for (int d = 0; d + 1 < W.D; ++d)
           ok = ok && axis_dft_smem<R>(dft_axis(W, d, fwd), 32) <= (size_t)smem_max;
-        plane = plane &&
-                plane_dft_smem<R>(dft_axis(W, W.D - 2, fwd), b, 1) <= (size_t)smem_max;
+        plane = plane && plane_dft_smem<R>(dft_axis(W, W.D - 2, fwd), b, 1) <= third;
       }
       if (ok) win_dft[w] = plane ? 2 : 1;
     }

@@ -154,8 +154,9 @@ def _space_ms(sv, dtype, generic):
     return ms
 
 
-# space shape, windows, type: padded 3 x 3
-SPEED = [((60, 60), (2, 2), np.float32), ((60, 60), (2, 2), np.float64)]
+# space shape, windows, type: padded 3 x 3, 100 x 100 (a plane fills an SM)
+SPEED = [((60, 60), (2, 2), np.float32), ((60, 60), (2, 2), np.float64),
+         ((80, 80), (80, 80), np.float32)]
 
 
 @pytest.mark.parametrize("space,windows,dtype", SPEED)
