@@ -1006,24 +1006,27 @@ class Engine {
     x.kpad = (x.P / 2 + kDftTk<R>) / kDftTk<R> * kDftTk<R>;
     x.n_in = fwd ? W.P[d] : W.L[d];
     x.n_out = fwd ? W.L[d] : W.P[d];
-    x.run = W.D > 1 ? dft_run(x.P) : 0;
+    x.lines = W.D > 1 ? dft_lines(x.P) : 4;
+    x.run = x.lines == 2 && x.P >= 40 ? 8 : 4;
     return x;
   }
 
-  // Terms of a run of the table DFT's sums (0: one sum).  One sum is at least
-  // as accurate as the radix passes below 24 points (errors of both
-  // directions within 1 % of theirs, or smaller) and where a large prime
-  // makes them sum directly too: primes (0.78 to 0.95 times their error),
-  // twice a prime (0.90 to 0.98).  Elsewhere it is up to 1.4 times as far
-  // off (P = 128; 1.02 at 30, 1.11 at 60, 1.19 at 80), in runs 0.83 to 1.0
-  // times.  Windows with one space axis had one sum per output before the
-  // other axes came to these kernels and keep it.
-  static int dft_run(int P) {
+  // Lines per tile of the table DFTs, which decides how their sums run: 4 one
+  // sum, 2 in runs, 1 in runs and groups of runs.  One sum is at least as
+  // accurate as the radix passes below 24 points (errors of both directions
+  // within 1 % of theirs, or smaller) and where a large prime makes them sum
+  // directly too: primes (0.78 to 0.95 times their error), twice a prime (0.90
+  // to 0.98).  Elsewhere it is up to 1.4 times as far off (P = 128; 1.02 at 30,
+  // 1.11 at 60, 1.19 at 80), in runs 0.83 to 1.0 times, but for the radix
+  // passes' most accurate lengths, 2^a 3^b from 54 on (1.01 at 54, 1.02 at 64
+  // and 108, 1.04 at 128).  Windows with one space axis had one sum per output
+  // before the other axes came to these kernels and keep it.
+  static int dft_lines(int P) {
     int largest = 1;  // prime factor
     for (int n = P, p = 2; n > 1; ++p)
       for (; n % p == 0; n /= p) largest = p;
-    if (P < 24 || P / largest < 3) return 0;
-    return P < 40 ? 4 : 8;
+    if (P < 24 || P / largest < 3) return 4;
+    return largest <= 3 && P >= 54 ? 1 : 2;
   }
 
   // Table-DFT jobs, tables and batch lists (windows marked in win_dft).
@@ -1156,9 +1159,8 @@ class Engine {
 
   // Warp iterations of the product loop over n_lines lines of one axis.
   static double dft_warp_work(const DftAxis<R> &x, int n_lines) {
-    const int tl = dft_tile_lines(x.run);
-    const int tiles = (n_lines + tl - 1) / tl * (x.kpad / kDftTk<R>);
-    return (double)((tiles + 31) / 32) * (x.H + 6) * (tl == 2 ? 0.6 : 1.0);
+    const int tiles = (n_lines + x.lines - 1) / x.lines * (x.kpad / kDftTk<R>);
+    return (double)((tiles + 31) / 32) * (x.H + 6) * (0.2 + 0.2 * x.lines);
   }
 
   // Planes per batch of every job: the number with the least warp work per
@@ -1196,8 +1198,7 @@ class Engine {
     const long resident = (sizeof(R) == sizeof(float) ? 512 : 384) / line_nt * (long)n_sm;
     const long cap = std::max<long>(4, (total / resident + 4) / 4 * 4);
     for (auto &j : jobs) {
-      const long tl = dft_tile_lines(j.b.run);
-      long nl = std::min<long>(tl * (line_nt / (j.b.kpad / kDftTk<R>)), cap);
+      long nl = std::min<long>(j.b.lines * (line_nt / (j.b.kpad / kDftTk<R>)), cap);
       while (nl > 4 && line_dft_smem<R>(j.b, nl) > dft_budget(line_nt)) nl -= 4;
       j.np = (int)std::max<long>(4, nl);
     }

@@ -64,7 +64,8 @@ template <typename R>
 struct DftAxis {
   const R *tab;
   int P, H, kpad, n_in, n_out;
-  int run;  // terms summed before they are added to the total (0: one sum)
+  int lines;  // lines of a thread's tile: 4 (one sum), 2 (runs) or 1 (runs of runs)
+  int run;    // terms of a run
 };
 
 // One window's planes: rows along axis b (contiguous), columns along axis a
@@ -94,10 +95,6 @@ struct AxisDftJob {
 // output pairs per thread: registers for 4 x 4 packed floats, 4 x 2 doubles
 template <typename R>
 constexpr int kDftTk = sizeof(R) == sizeof(float) ? 4 : 2;
-
-// lines per thread's tile: 4, or 2 where the sums run in two levels, whose
-// totals take the registers of the other two lines
-__host__ __device__ inline int dft_tile_lines(int run) { return run > 0 ? 2 : 4; }
 
 __host__ __device__ inline int dft_round4(int n) { return (n + 3) & ~3; }
 
@@ -194,14 +191,17 @@ __device__ __forceinline__ void dft_load_table(R *to, const DftAxis<R> &x) {
   for (int e = threadIdx.x; e < n; e += NT) cp_async<16>(to + e * per, x.tab + e * per);
 }
 
-// Accumulators of a tile of TL lines x TK output pairs; with TL = 2, the
-// totals of the runs before this one.
+// Accumulators of a tile of TL lines x TK output pairs; with TL = 2, also the
+// totals of the runs before this one; with TL = 1, those of this group of
+// kDftGroup runs and of the groups before it.
+constexpr int kDftGroup = 4;
 template <typename R, int TL>
 struct DftTile {
   static constexpr int TK = kDftTk<R>;
-  static constexpr bool kTwo = TL == 2;
+  static constexpr bool kRuns = TL < 4, kGroups = TL == 1;
   Cx<R> a[TL][TK], b[TL][TK];
-  Cx<R> ta[kTwo ? TL : 1][TK], tb[kTwo ? TL : 1][TK];
+  Cx<R> ta[kRuns ? TL : 1][TK], tb[kRuns ? TL : 1][TK];
+  Cx<R> ga[TK], gb[TK];  // groups
 
   // from x_0 and x_{P/2} (k0 is even: the sign of x_{P/2} follows m)
   __device__ __forceinline__ void start(const Cx<R> (&u)[TL], const Cx<R> (&v)[TL]) {
@@ -211,7 +211,8 @@ struct DftTile {
       for (int m = 0; m < TK; ++m) {
         a[i][m] = (m & 1) ? csub(u[i], v[i]) : cadd(u[i], v[i]);
         b[i][m] = cmake<Cx<R>>((R)0, (R)0);
-        if constexpr (kTwo) ta[i][m] = tb[i][m] = b[i][m];
+        if constexpr (kRuns) ta[i][m] = tb[i][m] = b[i][m];
+        if constexpr (kGroups) ga[m] = gb[m] = b[i][m];
       }
   }
   // one pair (s, d) of each line, with the table values at c, n
@@ -244,6 +245,15 @@ struct DftTile {
         b[i][m] = cscale(d[i], nv[m]);
       }
   }
+  // the group's sums into the totals; a new group
+  __device__ __forceinline__ void end_group() {
+#pragma unroll
+    for (int m = 0; m < TK; ++m) {
+      ga[m] = cadd(ga[m], ta[0][m]);
+      gb[m] = cadd(gb[m], tb[0][m]);
+      ta[0][m] = tb[0][m] = cmake<Cx<R>>((R)0, (R)0);
+    }
+  }
   __device__ __forceinline__ void finish() {
 #pragma unroll
     for (int i = 0; i < TL; ++i)
@@ -251,6 +261,10 @@ struct DftTile {
       for (int m = 0; m < TK; ++m) {
         a[i][m] = cadd(ta[i][m], a[i][m]);
         b[i][m] = cadd(tb[i][m], b[i][m]);
+        if constexpr (kGroups) {
+          a[i][m] = cadd(ga[m], a[i][m]);
+          b[i][m] = cadd(gb[m], b[i][m]);
+        }
       }
   }
   // outputs k0 .. of line i at out + k * ks, k < n_out
@@ -296,7 +310,7 @@ __device__ __forceinline__ void dft_accumulate_raw(DftTile<R, TL> &acc,
                                                    const Cx<R> *const (&lo)[TL], int es,
                                                    const DftAxis<R> &x, const R *tab, int k0) {
   using C = Cx<R>;
-  constexpr bool kTwo = TL == 2;
+  constexpr bool kRuns = TL < 4;
   const int mid = x.P / 2;
   const bool has_mid = x.P % 2 == 0 && mid < x.n_in;
   const int both = min(x.P - x.n_in, x.H);  // pairs 1 .. both have one member
@@ -319,7 +333,7 @@ __device__ __forceinline__ void dft_accumulate_raw(DftTile<R, TL> &acc,
       else
         u[i] = v[i] = lo[i][e];
     }
-    if constexpr (kTwo) {
+    if constexpr (kRuns) {
       if (new_run)
         acc.add_new_run(u, v, cj, nj);
       else
@@ -333,32 +347,30 @@ __device__ __forceinline__ void dft_accumulate_raw(DftTile<R, TL> &acc,
     cj += x.kpad;
     nj += x.kpad;
   };
-  if constexpr (kTwo) {
-    // the pairs with one member, then those with both, in runs
+  if constexpr (kRuns) {
     int end = x.run;  // last pair of the run
     bool fresh = false;
-    while (j <= both) {
-      const int stop = min(both, end);
-      term(false, fresh);
-      fresh = false;
+    [[maybe_unused]] int runs = 0;
+    // the pairs up to last, in runs
+    auto terms = [&](int last, bool both_in) {
+      while (j <= last) {
+        const int stop = min(last, end);
+        if constexpr (TL == 1) {
+          if (fresh && runs % kDftGroup == 1 && runs > 1) acc.end_group();
+        }
+        term(both_in, fresh);
+        fresh = false;
 #pragma unroll 2
-      while (j <= stop) term(false, false);
-      if (j > end) {
-        end += x.run;
-        fresh = true;
+        while (j <= stop) term(both_in, false);
+        if (j > end) {
+          end += x.run;
+          ++runs;
+          fresh = true;
+        }
       }
-    }
-    while (j <= x.H) {
-      const int stop = min(x.H, end);
-      term(true, fresh);
-      fresh = false;
-#pragma unroll 2
-      while (j <= stop) term(true, false);
-      if (j > end) {
-        end += x.run;
-        fresh = true;
-      }
-    }
+    };
+    terms(both, false);
+    terms(x.H, true);
     acc.finish();
   } else {
 #pragma unroll 1
@@ -397,10 +409,12 @@ template <typename R, bool FWD, typename InAt, typename OutAt, typename I>
 __device__ __forceinline__ void dft_from_raw(const Cx<R> *raw, int es, int n_lines,
                                              const DftAxis<R> &x, const R *tab, InAt in_at,
                                              OutAt out_at, I ks) {
-  if (x.run > 0)
+  if (x.lines == 4)
+    dft_tiles_from_raw<R, FWD, 4>(raw, es, n_lines, x, tab, in_at, out_at, ks);
+  else if (x.lines == 2)
     dft_tiles_from_raw<R, FWD, 2>(raw, es, n_lines, x, tab, in_at, out_at, ks);
   else
-    dft_tiles_from_raw<R, FWD, 4>(raw, es, n_lines, x, tab, in_at, out_at, ks);
+    dft_tiles_from_raw<R, FWD, 1>(raw, es, n_lines, x, tab, in_at, out_at, ks);
 }
 
 // The transforms of n rows of shared memory (elements side by side, rows rs
@@ -439,10 +453,12 @@ __device__ __forceinline__ void dft_tiles_in_place(Cx<R> *rows, int rs, int n,
 template <typename R, bool FWD, int NT>
 __device__ __forceinline__ void dft_rows_in_place(Cx<R> *rows, int rs, int n,
                                                   const DftAxis<R> &x, const R *tab) {
-  if (x.run > 0)
+  if (x.lines == 4)
+    dft_tiles_in_place<R, FWD, NT, 4>(rows, rs, n, x, tab);
+  else if (x.lines == 2)
     dft_tiles_in_place<R, FWD, NT, 2>(rows, rs, n, x, tab);
   else
-    dft_tiles_in_place<R, FWD, NT, 4>(rows, rs, n, x, tab);
+    dft_tiles_in_place<R, FWD, NT, 1>(rows, rs, n, x, tab);
 }
 
 // Finished rows of shared memory (stride rs) to n rows of n_out values at

@@ -103,7 +103,8 @@ def test_plane_batch_matches_separate_solves():
             assert rel_l2(o, r) <= 1e-5
 
 
-@pytest.mark.parametrize("length", [24, 35, 48, 64, 70, 100])  # padded 30, 44, 60, 80, 88, 125
+# padded 30, 44, 60, 64, 80, 88, 108, 125
+@pytest.mark.parametrize("length", [24, 35, 48, 51, 64, 70, 86, 100])
 def test_no_less_accurate_than_the_radix_passes(length):
     """Smooth padded lengths: both directions of a square window against the
     double operators, with the table DFTs and with the generic passes (the
