@@ -986,7 +986,7 @@ class Engine {
           ok = ok && axis_dft_smem<R>(dft_axis(W, d, fwd), 32) <= (size_t)smem_max;
         plane = plane && plane_dft_smem<R>(dft_axis(W, W.D - 2, fwd), b, 1) <= third;
       }
-      if (ok) win_dft[w] = plane ? 2 : 1;
+      if (ok && dft_is_faster(W, plane)) win_dft[w] = plane ? 2 : 1;
     }
     n_generic = 0;
     max_d_generic = 0;
@@ -1027,6 +1027,43 @@ class Engine {
       for (; n % p == 0; n /= p) largest = p;
     if (P < 24 || P / largest < 3) return 4;
     return largest <= 3 && P >= 54 ? 1 : 2;
+  }
+
+  // Time of an axis, forward and adjoint, in us per million values, fitted to
+  // square planes of 2 x 2 to 128 x 128 points: of the table products, and of
+  // the radix passes, which sum directly over prime factors above 5.
+  static double dft_table_us(int P) {
+    const bool f = sizeof(R) == sizeof(float);
+    switch (dft_lines(P)) {
+      case 4: return f ? 3.5 + 0.155 * P : 6.0 + 0.38 * P;
+      case 2: return f ? 4.5 + 0.16 * P : 5.0 + 0.45 * P;
+      default: return f ? 3.0 + 0.25 * P : 0.8 * P;
+    }
+  }
+  static double dft_radix_us(int P) {
+    int largest = 1;  // prime factor
+    for (int n = P, p = 2; n > 1; ++p)
+      for (; n % p == 0; n /= p) largest = p;
+    const bool f = sizeof(R) == sizeof(float);
+    if (largest <= 5) return f ? 29.0 : 35.0;
+    if (f || largest > 13) return 1e9;
+    return P == largest ? 46.0 : largest == 7 ? 52.0 : 60.0;
+  }
+  // A window of several axes goes to the table products where they take less
+  // time than the radix passes: in float all but planes of 108 and more points
+  // 2^a 3^b (128 x 128: 1030 us, radix passes 928), in double, whose
+  // arithmetic bounds them, up to about 70 points of smooth lengths (60 x 60:
+  // 1602 and 1972 us, 75 x 75: 1157 and 1063, 125 x 125: 1762 and 982).  An
+  // axis of its own pass takes at least its memory traffic.
+  static bool dft_is_faster(const WindowPlan &W, bool plane) {
+    if (W.D == 1) return true;
+    double table = 0.0, radix = 0.0;
+    for (int d = 0; d < W.D; ++d) {
+      const double own = sizeof(R) == sizeof(float) ? 10.0 : 20.0;
+      table += plane ? dft_table_us(W.P[d]) : std::max(own, dft_table_us(W.P[d]));
+      radix += dft_radix_us(W.P[d]);
+    }
+    return table < radix;
   }
 
   // Table-DFT jobs, tables and batch lists (windows marked in win_dft).

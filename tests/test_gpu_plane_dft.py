@@ -155,9 +155,12 @@ def _space_ms(sv, dtype, generic):
     return ms
 
 
-# space shape, windows, type: padded 3 x 3, 100 x 100 (a plane fills an SM)
+# space shape, windows, type: padded 3 x 3, 100 x 100 (a plane fills an SM),
+# 128 x 128, 75 x 75, 125 x 10
 SPEED = [((60, 60), (2, 2), np.float32), ((60, 60), (2, 2), np.float64),
-         ((80, 80), (80, 80), np.float32)]
+         ((80, 80), (80, 80), np.float32), ((102, 102), (102, 102), np.float32),
+         ((102, 102), (102, 102), np.float64), ((60, 60), (60, 60), np.float64),
+         ((100, 40), (100, 8), np.float64)]
 
 
 @pytest.mark.parametrize("space,windows,dtype", SPEED)
