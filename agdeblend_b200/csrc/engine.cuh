@@ -1205,13 +1205,14 @@ class Engine {
   // barriers and first loads), within a block's share of the shared memory
   // and small enough that the batches fill the device.  The smallest planes
   // take the most: 3 x 3, 47.5 M values, forward and adjoint together 2352 us
-  // in batches of 32, 831 in 128 (5 x 5, 32.1 M: 728 and 389, 497 in 256);
-  // radix passes 1481 and 953.
+  // in batches of 32, 831 in 128 (5 x 5, 32.1 M: 728 and 389, 497 in 256;
+  // 10 x 10, 32.2 M: 439 in 32, 473 in 64); radix passes 1481, 953 and 1183.
   void pick_plane_batches(std::vector<PlaneDftJob<R>> &jobs) const {
     long total = 0;
     for (const auto &j : jobs) total += j.planes;
-    const long most = std::min<long>(128, std::max<long>(1, total / (4L * n_sm)));
     for (auto &j : jobs) {
+      const long cap = std::min(128, std::max(32, 3200 / (j.a.P * j.b.P)));
+      const long most = std::min<long>(cap, std::max<long>(1, total / (4L * n_sm)));
       double best = 1e300;
       j.np = 1;
       for (int np = 1; np <= most; ++np) {
