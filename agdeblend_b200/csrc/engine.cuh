@@ -316,6 +316,13 @@ class Engine {
     return true;
   }
 
+  static int largest_prime(int n) {
+    int largest = 1;
+    for (int p = 2; n > 1; ++p)
+      for (; n % p == 0; n /= p) largest = p;
+    return largest;
+  }
+
   static void pfa_strides(PfaShape &sh) {
     int g = 1;
     for (int i = sh.nf - 1; i >= 0; --i) {
@@ -396,16 +403,22 @@ class Engine {
   }
 
   // Transform shape of every window, and the largest factor and length.
-  // False when some window has none that fits in shared memory (traces of
-  // over about 14,000 samples, 7,000 in double): the generic kernel serves
-  // all of them then.  wav_padded: some trace length is not itself a
-  // product of supported factors.
+  // False when some window has none that fits in shared memory (padded traces
+  // of over 13,464 samples, 6,732 in double), and when all lengths without a
+  // transform of their own are products of primes up to 19: the generic
+  // kernel serves all of them then.  Its radix passes are more accurate there
+  // than the padded transform, at 3 to 5 times the time (relative error of
+  // the operators at 512 samples 2.12e-7 and 2.26e-7, at 2048 2.18e-7 and
+  // 2.40e-7); with a larger prime it is the other way round (1472 = 64 * 23:
+  // 2.32e-7 and 2.28e-7, 1791 = 9 * 199: 3.82e-7 and 2.35e-7).  wav_padded:
+  // some trace length is not itself a product of supported factors.
   bool pick_wavelet_shapes(std::vector<PfaShape> &shapes, int &fmax, int &n_max) {
     const char *env = std::getenv("AGD_GPU_GENERIC");
     if (env != nullptr && env[0] == '1') return false;
     std::map<int, PfaShape> by_c;
     fmax = n_max = 1;
     wav_padded = false;
+    bool smooth = true;  // lengths to be padded: no prime above 19
     for (const WindowPlan &W : plan.windows) {
       auto it = by_c.find(W.C);
       if (it == by_c.end()) {
@@ -414,11 +427,15 @@ class Engine {
         it = by_c.emplace(W.C, sh).first;
       }
       const PfaShape &sh = it->second;
-      if (sh.N != W.C) wav_padded = true;
+      if (sh.N != W.C) {
+        wav_padded = true;
+        smooth = smooth && largest_prime(W.C) <= 19;
+      }
       for (int i = 0; i < sh.nf; ++i) fmax = std::max(fmax, sh.f[i]);
       n_max = std::max(n_max, sh.N);
       shapes.push_back(sh);
     }
+    if (wav_padded && smooth) return wav_padded = false;
     return (size_t)n_max * sizeof(C) <= (size_t)smem_max;
   }
 
@@ -1022,9 +1039,7 @@ class Engine {
   // and 108, 1.04 at 128).  Windows with one space axis had one sum per output
   // before the other axes came to these kernels and keep it.
   static int dft_lines(int P) {
-    int largest = 1;  // prime factor
-    for (int n = P, p = 2; n > 1; ++p)
-      for (; n % p == 0; n /= p) largest = p;
+    const int largest = largest_prime(P);
     if (P < 24 || P / largest < 3) return 4;
     return largest <= 3 && P >= 54 ? 1 : 2;
   }
@@ -1041,9 +1056,7 @@ class Engine {
     }
   }
   static double dft_radix_us(int P) {
-    int largest = 1;  // prime factor
-    for (int n = P, p = 2; n > 1; ++p)
-      for (; n % p == 0; n /= p) largest = p;
+    const int largest = largest_prime(P);
     const bool f = sizeof(R) == sizeof(float);
     if (largest <= 5) return f ? 29.0 : 35.0;
     if (f || largest > 13) return 1e9;
