@@ -31,8 +31,7 @@ namespace agd {
 // ------------------------------------------------------------ twiddle tables
 
 // Transform lengths with a constant twiddle table W_N^k = exp(-2 pi i k / N).
-constexpr int kTwSizes[] = {6,  7,  9,  10, 11, 12, 13,  15,  16, 17, 19, 20,
-                             23, 24, 25, 27, 32, 40, 48, 64, 80, 160, 320};
+constexpr int kTwSizes[] = {9, 16, 25, 27, 32, 160, 320};
 constexpr int kNumTw = (int)(sizeof(kTwSizes) / sizeof(int));
 
 __host__ __device__ constexpr int tw_offset(int n) {
@@ -54,10 +53,6 @@ constexpr int kTwTotal = tw_total();
 
 static __constant__ float2 c_tw_f[kTwTotal];
 static __constant__ double2 c_tw_d[kTwTotal];
-
-// Never launched: an attribute of it marks a context whose tables are filled.
-template <typename R>
-__global__ void tables_mark() {}
 
 template <typename R>
 __device__ __forceinline__ Cx<R> ctw(int idx);
@@ -113,11 +108,6 @@ __device__ __forceinline__ void prefetch_l2(const void *p, long n) {
 }
 
 // ------------------------------------------------------------ register DFTs
-
-template <bool INV, typename C>
-__device__ __forceinline__ C mul_i(C a) {  // -i a (forward) or +i a (inverse)
-  return INV ? cmake<C>(-a.y, a.x) : cmake<C>(a.y, -a.x);
-}
 
 // a + r b and a - r b for r = -i (forward) or +i (inverse): the components
 // cross over, so these stay scalar (a packed form would need them swapped)
@@ -358,26 +348,8 @@ __device__ __forceinline__ void dft(Cx<R> (&v)[N]) {
   } else if constexpr (small_split(N) != 0) {
     constexpr int N1 = small_split(N);
     dft_fourstep<R, N1, N / N1, INV>(v);
-  } else if constexpr (N % 2 == 1) {
-    dft_odd<R, N, INV>(v);
   } else {
-    // prime length without a table: direct DFT (only small primes reach here)
-    static_assert(N <= 13, "unsupported register DFT length");
-    C out[N];
-#pragma unroll
-    for (int q = 0; q < N; ++q) {
-      C acc = v[0];
-#pragma unroll
-      for (int r = 1; r < N; ++r) {
-        R s, c;
-        sincospi((R)(2 * ((r * q) % N)) / (R)N, &s, &c);
-        const C w = cmake<C>(c, INV ? s : -s);
-        acc = cadd(acc, cmul(v[r], w));
-      }
-      out[q] = acc;
-    }
-#pragma unroll
-    for (int q = 0; q < N; ++q) v[q] = out[q];
+    dft_odd<R, N, INV>(v);
   }
 }
 

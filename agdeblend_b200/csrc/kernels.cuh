@@ -8,7 +8,7 @@
 //
 // Forward  A x : axis_pass (space IFFT per axis, crop P->L) -> time_c2r_ola
 //                (time c2r, taper, overlap-add) -> [wavelet_apply] ->
-//                blend_gather (ordered sum into the record, mute, residual)
+//                record_gather (ordered sum into the record, mute, residual)
 // Adjoint A^H r: time_r2c (blend adjoint gather, taper, time r2c, x2 bins)
 //                -> axis_pass (zero-pad L->P, space FFT per axis) with the
 //                ISTA update and soft threshold fused into the last pass.
@@ -36,6 +36,11 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+
+// Never launched: an attribute of it marks a context whose constant tables
+// (fast.cuh) are filled.
+template <typename R>
+__global__ void tables_mark() {}
 
 // ------------------------------------------------------------ job records
 
