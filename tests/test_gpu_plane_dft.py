@@ -169,3 +169,13 @@ def test_not_slower_than_the_radix_passes(space, windows, dtype):
     spread of the timing where both sides are the same kernels)."""
     sv = _survey(space, windows, nt=600, wt=128)
     assert _space_ms(sv, dtype, False) <= 1.1 * _space_ms(sv, dtype, True)
+
+
+def test_radix_passes_beside_table_products():
+    """In double, 60-trace axes (padded 75) keep the radix passes and 61-trace
+    ones (77 = 7 x 11) do not: windows of both kinds in one survey."""
+    sv = _survey((60, 121), (60, 60))
+    prob = A.Problem.from_survey(sv, np.float64)
+    assert prob.kernels()["space_fwd"] in ("plane_dft", "line_dft")
+    prob.close()
+    _check_operators(sv, np.float64, 1)
