@@ -865,7 +865,7 @@ class Engine {
       }
     } else {
       // double: two stages with one block per SM, and one-stage and pipelined
-      // kernels in blocks small enough for 255 registers per thread
+      // kernels in blocks small enough for 128 to 255 registers per thread
       if (shape_is<1, 40, 1, 1>(W)) {
         add_fwd<1, 40, 1, 1, 256, 128, 2, 1>(c);
         add_adj<1, 40, 1, 1, 192, 96, 2, 1>(c);

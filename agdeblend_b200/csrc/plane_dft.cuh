@@ -18,7 +18,7 @@
 // It is bound by the FP32 pipe and the issue slots around it (37 x 101
 // traces of 873 samples, planes of 23 x 44: 1.1 G multiply-adds, 30 us at
 // 36.7 T/s, against 37 us of memory traffic forward and 60 us adjoint;
-// measured 136 and 188 us, and 730 and 826 us by the generic block FFTs), so:
+// measured 152 and 193 us, and 730 and 826 us by the generic block FFTs), so:
 //
 //  * a thread accumulates 4 lines x 4 output pairs in registers (packed
 //    f32x2 multiply-adds on the (re, im) pairs: the same rate as scalar
@@ -41,8 +41,9 @@
 //  * the last two axes of a window are one kernel (plane_dft): the planes
 //    go axis by axis through shared memory, and the adjoint applies the
 //    ISTA update to the model rows on the way out.  Other axes (the first
-//    of a 3-D window; of two axes too long for a plane to fit in shared
-//    memory, the first) are one pass each over memory (axis_dft);
+//    of a 3-D window; of two axes too long for three planes to fit in an
+//    SM's shared memory, the first) are one pass each over memory
+//    (axis_dft);
 //  * persistent blocks of 128 threads, up to four per SM (registers), so
 //    that one block's barriers are covered by the others;
 //  * windows with one axis (line_dft): a batch is as many lines as the

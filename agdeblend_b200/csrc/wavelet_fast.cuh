@@ -39,7 +39,9 @@
 // back to sample t.  The cost is that of a transform of twice the length;
 // a length-C transform would need a direct DFT of its prime factor (199
 // products per sample).  13,230 traces of 1791 samples, both directions:
-// 59.8 ms with the direct factor-199 passes, 0.54 ms padded to N = 3696
+// 59.8 ms with the direct factor-199 passes, 0.47 ms padded to N = 3696.
+// Lengths whose radix passes sum directly over no prime above 19 keep them:
+// they are the more accurate there (engine.cuh, pick_wavelet_shapes).
 //
 // The adjoint reads its traces straight from the blended record (the blend
 // adjoint gather of src/blend.c:1262-1292), so the traces are not written

@@ -407,7 +407,7 @@ def measure_single(args, name, rank, world, local, cpu_its):
     # Algorithmic bytes per launch: the share of
     # B_iter = 3 M 8 + 4 R 4 each kernel is responsible for - the forward
     # space kernel reads the model once, the adjoint space kernel reads and
-    # writes it once, the blend gather writes A x and reads d, the adjoint
+    # writes it once, the record gather writes A x and reads d, the adjoint
     # time kernel reads the residual; the time-axis kernels move only
     # intermediates (0 algorithmic bytes).
     nf = int(prof[14])
@@ -450,8 +450,8 @@ def measure_single(args, name, rank, world, local, cpu_its):
     line = None
     if rank == 0:
         # kernels per iteration as the library counts them (space and time
-        # kernels both ways per window class, generic passes, the blend
-        # gather, the threshold-schedule step, wavelet kernels)
+        # kernels both ways per window class, generic passes, the record
+        # gather with the threshold-schedule step, wavelet kernels)
         launches = args.steps * int(info[14])
         line = {"metric": metric_of(name), "value": value, "unit": UNIT, "n_gpus": world,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_iter,
@@ -568,7 +568,7 @@ def measure_batch(args, name, rank, world, local):
     M, Rn = int(info[1]), int(info[2])
     peak, peak_kind = hbm_peak()
     phases = {"space_fwd": (prof[0], 8.0 * M), "time_fwd": (prof[1], 0.0),
-              "blend_gather": (prof[3], 8.0 * Rn), "time_adj": (prof[4], 4.0 * Rn),
+              "record_gather": (prof[3], 8.0 * Rn), "time_adj": (prof[4], 4.0 * Rn),
               "space_adj": (prof[5], 16.0 * M)}
     dom = max(phases, key=lambda k: phases[k][0])
     dom_ms, dom_bytes = phases[dom]

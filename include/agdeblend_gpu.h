@@ -46,13 +46,14 @@ void agd_gpu_problem_destroy(agd_gpu_problem *problem);
  * [8] 1 if the shape-specialised kernels serve every window, 2 if they
  * serve some, 0 if none, [9] 1 if the prime-factor wavelet kernel serves
  * the problem with transforms of the traces' own lengths (0: some are
- * zero-padded to a length it has, or the generic kernel serves them), [10] and [11] the space-kernel candidates picked by the
- * set-up timing for the forward and adjoint of the first window class (-1
- * without shape-specialised kernels), [12] and [13] that class's number of
+ * zero-padded to a length it has, or the generic kernel serves them), [10]
+ * and [11] the space-kernel candidates picked by the set-up timing for the
+ * forward and adjoint of the first window class (-1 without
+ * shape-specialised kernels), [12] and [13] that class's number of
  * candidates, [14] kernels launched per iteration, [15] window classes on
- * the shape-specialised kernels, [16] windows on them, [17] and [18] the
- * time-kernel candidates picked for the first time group (-1 without
- * one), [19] its number of candidates, [20] the wavelet-kernel candidate
+ * the shape-specialised kernels, [16] windows on them, [17] and [18] 0 and
+ * [19] 1 with windows on the trace-pair time kernels (one forward and one
+ * adjoint kernel, nothing to pick), -1, -1 and 0 without, [20] the wavelet-kernel candidate
  * picked (-1 without the prime-factor kernel), [21] their number, [22]
  * windows with one space axis on the table-DFT kernels (lengths without a
  * shape-specialised kernel, up to 128). */
