@@ -24,6 +24,7 @@
 #include <stdint.h>
 #include <type_traits>
 
+#include "const_trig.hpp"
 #include "kernels.cuh"
 
 namespace agd {
@@ -155,27 +156,7 @@ __host__ __device__ constexpr int crt_index(int k1, int k2, int N1, int N2) {
   return k;
 }
 
-// cos and sin of 2 pi m / n at compile time (Taylor series about 0 of an
-// angle in [0, pi], in double precision), so that the register DFTs of odd
-// length have literal coefficients.
-constexpr double const_cos(int m, int n) {
-  const double x = 6.283185307179586476925286766559 * m / n;
-  double term = 1.0, sum = 1.0;
-  for (int i = 1; i < 24; ++i) {
-    term *= -x * x / ((2.0 * i - 1.0) * (2.0 * i));
-    sum += term;
-  }
-  return sum;
-}
-constexpr double const_sin(int m, int n) {
-  const double x = 6.283185307179586476925286766559 * m / n;
-  double term = x, sum = x;
-  for (int i = 1; i < 24; ++i) {
-    term *= -x * x / ((2.0 * i) * (2.0 * i + 1.0));
-    sum += term;
-  }
-  return sum;
-}
+// Coefficients of an odd DFT.
 template <typename R, int N>
 struct OddTable {  // m = 0 .. (N - 1) / 2
   R c[(N + 1) / 2], s[(N + 1) / 2];
