@@ -40,6 +40,7 @@ class Engine {
   Plan plan;
   cudaStream_t stream = nullptr;
   int smem_max = 0;
+  int context = 0;  // number of the CUDA context (enter_context)
   FftTable<R> fft;
   DevArray<FftDesc> d_descs;
   DevArray<C> d_tw;
@@ -193,8 +194,9 @@ class Engine {
       CK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
       CK(cudaDeviceGetAttribute(&block_reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
     }
-    set_smem_limits();
     try {
+      context = enter_context();
+      set_smem_limits();
       build();
     } catch (...) {
       // nothing of this engine may still run when its arrays are released
@@ -224,13 +226,18 @@ class Engine {
   // own static shared memory; smem_max becomes the smallest such limit.
   template <typename K>
   int opt_in(K kernel, int limit) {
-    // set once per kernel and context: the attribute stays, and is asked for
-    // in the context itself, which a device reset replaces
+    // once per kernel and context: the attribute stays
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, int> done;
+    const std::pair<int, const void *> key(context, reinterpret_cast<const void *>(kernel));
+    std::lock_guard<std::mutex> lk(mu);
+    const auto it = done.find(key);
+    if (it != done.end()) return it->second;
     cudaFuncAttributes fa;
     CK(cudaFuncGetAttributes(&fa, kernel));
     const int dyn = limit - (int)fa.sharedSizeBytes;
-    if (fa.maxDynamicSharedSizeBytes != dyn)
-      CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+    if (context > 0) done[key] = dyn;
     return dyn;
   }
 
@@ -262,17 +269,34 @@ class Engine {
                            opt_in(wavelet_fast<R, 1, 32, PAD>, limit)});
   }
 
-  // twiddle tables of the register DFTs in constant memory of the current
-  // context (fast.cuh), shared by the fast space, time and wavelet kernels;
-  // filled once per context, which tables_mark's attribute tells (a device
-  // reset clears both)
-  void upload_twiddles() {
-    constexpr int kFilled = 65536;  // above the 48 KB that a kernel starts with
+  // Number of the current context, for what is set once per context; a new
+  // one gets the constant tables.  The context itself holds the number, as an
+  // attribute of tables_mark, because a device reset replaces the context
+  // without a word (asking every kernel for its attribute instead takes 30 us
+  // of a 0.9 ms call).  0 when the numbers are used up.
+  int enter_context() {
+    constexpr int kFirst = 65536, kStep = 1024;  // above the 48 KB that a kernel starts with
     static std::mutex mu;
+    static int last = 0;
     std::lock_guard<std::mutex> lk(mu);
-    cudaFuncAttributes fa;
-    CK(cudaFuncGetAttributes(&fa, tables_mark<R>));
-    if (fa.maxDynamicSharedSizeBytes == kFilled) return;
+    auto number = [&] {
+      cudaFuncAttributes fa;
+      CK(cudaFuncGetAttributes(&fa, tables_mark<R>));
+      return (fa.maxDynamicSharedSizeBytes - kFirst) / kStep;
+    };
+    const int known = number();
+    if (known > 0) return known;
+    upload_twiddles();
+    if (kFirst + (last + 1) * kStep > optin_smem()) return 0;
+    ++last;
+    CK(cudaFuncSetAttribute(tables_mark<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            kFirst + last * kStep));
+    return number() == last ? last : 0;
+  }
+
+  // twiddle tables of the register DFTs in constant memory of the current
+  // context (fast.cuh), shared by the fast space, time and wavelet kernels
+  void upload_twiddles() {
     std::vector<C> tw(kTwTotal);
     for (int i = 0, off = 0; i < kNumTw; off += kTwSizes[i], ++i)
       for (int k = 0; k < kTwSizes[i]; ++k) {
@@ -287,8 +311,6 @@ class Engine {
       CK(cudaMemcpyToSymbolAsync(c_tw_d, tw.data(), tw.size() * sizeof(C), 0,
                                  cudaMemcpyHostToDevice, stream));
     CK(cudaStreamSynchronize(stream));
-    CK(cudaFuncSetAttribute(tables_mark<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            kFilled));
   }
 
   // C = product of pairwise coprime prime powers with a register DFT; the
@@ -565,7 +587,6 @@ class Engine {
       j.C = W.C;
     }
     wavf_jobs.upload(jobs, stream);
-    upload_twiddles();
     // candidates: blocks per SM and pairs per block (about a third of the
     // SM's shared memory per block at three blocks)
     std::vector<WaveletCand> cands;
@@ -1837,7 +1858,6 @@ class Engine {
     setup_mark("buffers");
     if (!classes.empty() || !tgroups.empty()) {
       opt_in_classes();
-      upload_twiddles();
       for (auto &c : classes) build_class(*c);
       for (auto &g : tgroups) build_time_group(*g);
     }
