@@ -12,6 +12,7 @@ import os
 import numpy as np
 import pytest
 
+import agd_oracle as O
 import agdeblend_b200 as A
 from agdeblend_b200 import synthetic as S
 from conftest import rel_l2
@@ -179,3 +180,71 @@ def test_radix_passes_beside_table_products():
     assert prob.kernels()["space_fwd"] in ("plane_dft", "line_dft")
     prob.close()
     _check_operators(sv, np.float64, 1)
+
+
+def _fk_long(w, x=None, y=None):
+    """The oracle's fk_forward of x or fk_adjoint of y in extended precision."""
+    real = np.longdouble
+    nd = len(w.shape)
+    h = w.lt // 2
+    scale = ((real(w.scaler) * w.space_taper().astype(real))[None, :, None]
+             * w.tapers[-1].astype(real)[None, None, :])
+    crop = (slice(None), *(slice(0, n) for n in w.shape), slice(0, w.lt))
+    if x is not None:
+        u = np.fft.irfftn(x, s=w.padded, axes=tuple(range(1, nd + 2))) * real(np.prod(w.padded))
+        u = u[crop].reshape(w.n_tw, w.n_traces, w.lt) * scale
+        out = np.zeros((w.n_traces, w.conv), real)
+        for t in range(w.n_tw):
+            out[:, t * h: t * h + w.lt] += u[t]
+        return out
+    seg = np.stack([y[:, t * h: t * h + w.lt] for t in range(w.n_tw)]) * scale
+    u = np.zeros((w.n_tw, *w.padded), real)
+    u[crop] = seg.reshape(w.n_tw, *w.shape, w.lt)
+    out = np.fft.rfftn(u, axes=tuple(range(1, nd + 2)))
+    out[..., 1: 1 + (w.padded[-1] - 1) // 2] *= 2
+    return out
+
+
+@pytest.mark.skipif(np.finfo(np.longdouble).eps > 1e-18, reason="no extended precision")
+@pytest.mark.parametrize("length", [24, 36, 40, 48])  # padded 30, 45, 50, 60
+def test_double_no_less_accurate_than_the_radix_passes(length):
+    """As in float, against extended precision; shots that do not overlap."""
+    n, nt = length * length, 260
+    zero = np.zeros(n, np.int32)
+    sv = S.Survey("one window", [0], [3], [[length, length, 100]], [[0, 0]],
+                  [[length, length, nt]], [(3 * nt * np.arange(n)).astype(np.int64)], [zero],
+                  [zero], [np.zeros((length, length, nt))], [np.zeros((length, length, nt))], 4)
+    plan = O.make_plan(sv.volumes, sv.n_dims, sv.window_shapes, sv.coords, sv.shapes,
+                       sv.shottimes, sv.channels, sv.trace_types, None, None, None)
+    (w,) = plan.windows
+    rng = np.random.default_rng(length)
+    size = int(np.prod(w.model_shape))
+    m = rng.standard_normal(2 * size)
+    y = _fk_long(w, x=(m[0::2].astype(np.longdouble)
+                       + 1j * m[1::2].astype(np.longdouble)).reshape(w.model_shape))
+    rec = rng.standard_normal(plan.cfg.total)
+    traces = np.zeros((n, w.conv), np.longdouble)
+    fwd = np.zeros(plan.cfg.total, np.longdouble)
+    for i, (off, ts, k) in enumerate(w.blend):
+        traces[i, ts: ts + k] = rec[off: off + k]
+        fwd[off: off + k] += y[i, ts: ts + k]
+    adj = _fk_long(w, y=traces).reshape(-1)
+    errors = []
+    for generic in (False, True):
+        old = os.environ.get("AGD_GPU_GENERIC")
+        os.environ["AGD_GPU_GENERIC"] = "1" if generic else "0"
+        try:
+            p = A.Problem.from_survey(sv, np.float64)
+        finally:
+            if old is None:
+                os.environ.pop("AGD_GPU_GENERIC", None)
+            else:
+                os.environ["AGD_GPU_GENERIC"] = old
+        g = p.adjoint(rec)
+        g = g[0::2].astype(np.longdouble) + 1j * g[1::2].astype(np.longdouble)
+        f = p.forward(m).astype(np.longdouble)
+        p.close()
+        errors.append([float(np.sqrt(np.sum(abs(a - b) ** 2) / np.sum(abs(b) ** 2)))
+                       for a, b in ((g, adj), (f, fwd))])
+    for table, radix in zip(*errors):
+        assert table <= 1.01 * radix
