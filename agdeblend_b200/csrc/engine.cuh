@@ -1058,22 +1058,27 @@ class Engine {
   // 1.11 at 60, 1.19 at 80), in runs 0.83 to 1.0 times, but for the radix
   // passes' most accurate lengths, 2^a 3^b from 54 on (1.01 at 54, 1.02 at 64
   // and 108, 1.04 at 128).  Windows with one space axis had one sum per output
-  // before the other axes came to these kernels and keep it.
+  // before the other axes came to these kernels and keep it.  In double one
+  // sum is the more accurate everywhere, because the tables' angles are exact
+  // and the radix passes' twiddles' are not (2.9e-16 to 3.9e-16 up to 78
+  // points, radix passes 3.3e-16 to 6.4e-16).
   static int dft_lines(int P) {
+    if (sizeof(R) == sizeof(double)) return 4;
     const int largest = largest_prime(P);
     if (P < 24 || P / largest < 3) return 4;
     return largest <= 3 && P >= 54 ? 1 : 2;
   }
 
   // Time of an axis, forward and adjoint, in us per million values, fitted to
-  // square planes of 2 x 2 to 128 x 128 points: of the table products, and of
-  // the radix passes, which sum directly over prime factors above 5.
+  // planes of 2 x 2 to 128 x 128 points: of the table products (in double the
+  // longest lines fill the shared memory of a block in few lines), and of the
+  // radix passes, which sum directly over prime factors above 5.
   static double dft_table_us(int P) {
-    const bool f = sizeof(R) == sizeof(float);
+    if (sizeof(R) == sizeof(double)) return 6.0 + 0.38 * P + (P > 120 ? 12.0 : 0.0);
     switch (dft_lines(P)) {
-      case 4: return f ? 3.5 + 0.155 * P : 6.0 + 0.38 * P;
-      case 2: return f ? 4.5 + 0.16 * P : 5.0 + 0.45 * P;
-      default: return f ? 3.0 + 0.25 * P : 0.8 * P;
+      case 4: return 3.5 + 0.155 * P;
+      case 2: return 4.5 + 0.16 * P;
+      default: return 3.0 + 0.25 * P;
     }
   }
   static double dft_radix_us(int P) {
@@ -1086,8 +1091,8 @@ class Engine {
   // A window of several axes goes to the table products where they take less
   // time than the radix passes: in float all but planes of 108 and more points
   // 2^a 3^b (128 x 128: 1030 us, radix passes 928), in double, whose
-  // arithmetic bounds them, up to about 70 points of smooth lengths (60 x 60:
-  // 1602 and 1972 us, 75 x 75: 1157 and 1063, 125 x 125: 1762 and 982).  An
+  // arithmetic bounds them, up to about 75 points of smooth lengths (60 x 60:
+  // 1370 and 1972 us, 75 x 75: 1020 and 1063, 125 x 125: 1760 and 982).  An
   // axis of its own pass takes at least its memory traffic.
   static bool dft_is_faster(const WindowPlan &W, bool plane) {
     if (W.D == 1) return true;

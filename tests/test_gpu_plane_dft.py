@@ -173,9 +173,9 @@ def test_not_slower_than_the_radix_passes(space, windows, dtype):
 
 
 def test_radix_passes_beside_table_products():
-    """In double, 60-trace axes (padded 75) keep the radix passes and 61-trace
-    ones (77 = 7 x 11) do not: windows of both kinds in one survey."""
-    sv = _survey((60, 121), (60, 60))
+    """In double, 64-trace axes (padded 80) keep the radix passes and 65-trace
+    ones (82 = 2 x 41) do not: windows of both kinds in one survey."""
+    sv = _survey((64, 129), (64, 64))
     prob = A.Problem.from_survey(sv, np.float64)
     assert prob.kernels()["space_fwd"] in ("plane_dft", "line_dft")
     prob.close()
